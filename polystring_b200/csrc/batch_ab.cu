@@ -66,16 +66,12 @@ BatchAB::BatchAB(const std::vector<ModelABParams>& ps, const std::vector<ModelAB
         // persistent sweeps where the grid has one, grouped line passes for the rest
         std::vector<int> swept, passes;
         for (int k = 0; k < (int)m_.size(); k++) {
-            if (m_[k]->persistent_sweep64()) own_.push_back(k);
-            else if (m_[k]->persistent_sweep()) swept.push_back(k);
-            else passes.push_back(k);
+            (m_[k]->persistent_sweep() ? swept : passes).push_back(k);
         }
-        // triblocks likewise (their own 64^3 sweep, their grids' generic sweep,
-        // else grouped line passes)
+        // triblocks likewise
         for (int j = 0; j < (int)t_.size(); j++) {
             const int k = (int)m_.size() + j;
-            if (t_[j]->persistent_sweep64()) own_.push_back(k);
-            else (t_[j]->persistent_sweep() ? swept : passes).push_back(k);
+            (t_[j]->persistent_sweep() ? swept : passes).push_back(k);
         }
         build_sweeps(swept);
         // groups: same number of long axes (the step's pass sequence) and the
@@ -140,8 +136,13 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
     }
     for (auto& kv : by_shape) {
         const int Lx = kv.first[0], Ly = kv.first[1], Lz = kv.first[2];
-        const int resident = sweep_desc_prepare(Lx, Ly, Lz);
-        const int tasks = sweep_tasks_per_phase(Lx, Ly, Lz);
+        auto descriptor = [&](int k) {
+            return k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
+        };
+        int nfrag = 0;
+        for (int k : kv.second) nfrag = std::max(nfrag, descriptor(k).nfrag);
+        const int resident = real_sweep_prepare(Lx, Ly, Lz, nfrag, true);
+        const int tasks = real_sweep_tasks(Lx, Ly, Lz);
         // A launch of n solves gives each per = resident / n CTAs (at most the
         // tasks of a phase) and lasts its longest solve's Ns steps, each step
         // sweep_rounds_per_step(per) rounds of tasks.  With the solves in
@@ -150,13 +151,13 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
         std::vector<int> ks = kv.second;
         std::stable_sort(ks.begin(), ks.end(), [&](int a, int b) { return Ns_of(a) > Ns_of(b); });
         const int nk = (int)ks.size();
-        auto per_of = [&](int n) { return std::max(1, std::min(tasks, resident / n)); };
+        auto per_of = [&](int n) { return std::max(1, std::min(tasks, resident / 2 / n)); };
         std::vector<double> best(nk + 1, 0.0);
         std::vector<int> from(nk + 1, 0);
         for (int i = 1; i <= nk; i++) {
             best[i] = -1.0;
-            for (int j = std::max(0, i - resident); j < i; j++) {
-                const double c = best[j] + (double)Ns_of(ks[j]) * sweep_rounds_per_step(Lx, Ly, Lz, per_of(i - j));
+            for (int j = std::max(0, i - resident / 2); j < i; j++) {
+                const double c = best[j] + (double)Ns_of(ks[j]) * real_sweep_step_cost(Lx, Ly, Lz, per_of(i - j));
                 if (best[i] < 0.0 || c < best[i]) { best[i] = c; from[i] = j; }
             }
         }
@@ -167,21 +168,19 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
             const size_t i0 = (size_t)run.first;
             chunks_.emplace_back();
             SweepChunk& c = chunks_.back();
-            c.Lx = Lx; c.Ly = Ly; c.Lz = Lz;
+            c.Lx = Lx; c.Ly = Ly; c.Lz = Lz; c.nfrag = nfrag;
             c.n = run.second - run.first;
             c.per = per_of(c.n);
             PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * (size_t)c.n));
-            std::vector<SweepArgs> d(c.n);
+            std::vector<RealProblem> d(c.n);
             for (int i = 0; i < c.n; i++) {
-                const int k = ks[i0 + i];
-                d[i] = k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
+                d[i] = descriptor(ks[i0 + i]);
                 d[i].bar = c.bar + 32 * (size_t)i;
-                d[i].twx = twiddle_table(Lx);
-                d[i].twy = twiddle_table(Ly);
-                d[i].twz = twiddle_table(Lz);
+                d[i].cta0 = 2 * i * c.per;
+                d[i].ncta = c.per;
             }
-            PS_CUDA(cudaMalloc(&c.dev, sizeof(SweepArgs) * d.size()));
-            PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(SweepArgs) * d.size(), cudaMemcpyHostToDevice));
+            PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
+            PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
         }
     }
 }
@@ -262,12 +261,7 @@ void BatchAB::enqueue_iteration() {
     int launches = 0;
     for (const SweepChunk& c : chunks_) {
         PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-        sweep_launch_desc(c.dev, c.Lx, c.Ly, c.Lz, c.per, c.n, st_);
-        launches++;
-    }
-    for (int k : own_) {
-        if (k < (int)m_.size()) m_[k]->enqueue_propagate(st_);
-        else t_[k - (int)m_.size()]->enqueue_propagate(st_);
+        real_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.Lz, c.nfrag, 2 * c.per * c.n, st_);
         launches++;
     }
     int Ns_max = 0;

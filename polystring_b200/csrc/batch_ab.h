@@ -43,8 +43,8 @@ private:
     // solves of one shape with a generic persistent sweep, in one cooperative
     // launch: n descriptors on the device, per CTAs a solve, n x 32 barrier words
     struct SweepChunk {
-        int Lx = 0, Ly = 0, Lz = 0, per = 0, n = 0;
-        SweepArgs* dev = nullptr;
+        int Lx = 0, Ly = 0, Lz = 0, nfrag = 0, per = 0, n = 0;
+        RealProblem* dev = nullptr;
         unsigned* bar = nullptr;
     };
     void build_group(Group& g);
@@ -58,7 +58,6 @@ private:
     std::vector<ModelABC*> t_;
     std::vector<Group> groups_;
     std::vector<SweepChunk> chunks_;
-    std::vector<int> own_;                   // solves propagated by their own 64^3 sweep (AB and ABC indices)
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t graph_ = nullptr;
     int launches_ = 0, launches_prop_ = 0;

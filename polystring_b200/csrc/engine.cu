@@ -117,6 +117,21 @@ std::vector<double> k2_orthogonal(const Cell& c, int Lx, int Ly, int Lz) {
     return k2;
 }
 
+void axis_k2(const Cell& c, double k[3]) {
+    const double PI = 3.14159265358979323846;
+    for (int d = 0; d < 3; d++) k[d] = d < c.dim ? -4.0 * PI * PI / (c.l[d] * c.l[d]) : 0.0;
+}
+
+// the shape matrix is diagonal (to the rounding of cos(pi / 2)), so |q|^2 of
+// k_laplacian is the sum of the axes' terms and its 27-image minimum the minimum
+// of each; the diagonal then holds 2 pi over the cell lengths
+bool cell_separable(const Cell& c) {
+    for (int r = 0; r < c.dim; r++)
+        for (int q = 0; q < c.dim; q++)
+            if (r != q && std::fabs(c.g[3 * r + q]) > 1e-14 * std::fabs(c.g[3 * r + r])) return false;
+    return true;
+}
+
 std::vector<double> k_laplacian(const Cell& c, int Na, int Nb, int Nc, double ds) {
     std::vector<double> out((size_t)Na * Nb * Nc);
     for (int i = 0; i < Na; i++)
@@ -421,43 +436,15 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
         }
         chain_->set_tables(L1, L2);
     }
+    // 3D grids of orthogonal cells propagate by the persistent sweep on real
+    // line operators (PS_B200_LINE_PASSES=1 keeps the line passes)
     const char* force = getenv("PS_B200_LINE_PASSES");
-    const char* generic = getenv("PS_B200_GENERIC_SWEEP");
-    const bool allow = !(force && force[0] == '1');
-    use_sweep64_ = allow && p.mde == 0 && sweep64_supported(p.Lx, p.Ly, p.Lz) && !(generic && generic[0] == '1');
-    // the 64^3 sweep needs its clusters resident (74 two-CTA clusters on a
-    // 148-SM B200); where fewer fit, the generic sweep runs the grid
-    if (use_sweep64_) {
-        sweep_grid_ = sweep64_prepare();
-        use_sweep64_ = sweep_grid_ > 0;
-    }
-    use_sweep_ = allow && p.mde == 0 && !use_sweep64_ && sweep_supported(p.Lx, p.Ly, p.Lz);
-    if (use_sweep64_) {
-        swZ_.alloc(6 * (size_t)M_);
-        const std::vector<double> tab = sweep64_axis_tables(p_.cell.l, dsA_);
-        swTab_.alloc(tab.size());
-        PS_CUDA(cudaMemcpy(swTab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMalloc(&swbar_, 64 * sizeof(unsigned)));
-        PS_CUDA(cudaMalloc(&swerr_, sizeof(int)));
-        PS_CUDA(cudaMemset(swerr_, 0, sizeof(int)));
-    }
-    if (use_sweep_) {
-        sweep_grid_ = sweep_prepare(p.Lx, p.Ly, p.Lz);
-        swZ_.alloc(6 * (size_t)M_);
-        swU_.alloc(2 * (size_t)M_);
-        std::vector<double> k2 = k2_orthogonal(p_.cell, p.Lx, p.Ly, p.Lz);
-        std::vector<double> L1(M_), L2(M_);
-        for (long m = 0; m < M_; m++) {
-            L1[m] = exp(dsA_ * k2[m]);
-            L2[m] = exp(0.5 * dsA_ * k2[m]);
-        }
-        swL1_.alloc(M_);
-        swL2_.alloc(M_);
-        PS_CUDA(cudaMemcpy(swL1_.p, L1.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMemcpy(swL2_.p, L2.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMalloc(&swbar_, 32 * sizeof(unsigned)));
-        PS_CUDA(cudaMalloc(&swerr_, sizeof(int)));
-        PS_CUDA(cudaMemset(swerr_, 0, sizeof(int)));
+    if (!(force && force[0] == '1') && (p.mde == 0 || (p.mde == 1 && cell_separable(p_.cell))) &&
+        real_sweep_supported(p.Lx, p.Ly, p.Lz)) {
+        const int n[3] = {p.Lx, p.Ly, p.Lz};
+        double k[3];
+        axis_k2(p_.cell, k);
+        real_ = new RealSweep(n, k, dsA_, 2, p.mde == 1);
     }
     hf_.alloc((size_t)(Ns_ + 1) * M_);
     hc_.alloc((size_t)(Ns_ + 1) * M_);
@@ -480,13 +467,14 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     launch_fill(hf_.p, M_, 1.0, st_);
     launch_fill(hc_.p, M_, 1.0, st_);
     launch_fill(yita_.p, M_, 0.0, st_);
-    if (!use_sweep_ && !use_sweep64_ && !batch_member) chain_->autotune(st_);
-    if (use_sweep_) {
-        sweep_variant_ = sweep_default_variant(p.Lx, p.Ly, p.Lz);
-        if (!batch_member) tune_sweep();
+    if (!real_ && !batch_member) chain_->autotune(st_);
+    if (real_ && !batch_member) {
+        // finite data for the timed sweeps (set_fields overwrites the factors)
+        for (double* f : {eFA_.p, eHA_.p, eFB_.p, eHB_.p}) launch_fill(f, M_, 1.0, st_);
+        real_->tune(sweep_descriptor(), st_);
     }
     PS_CUDA(cudaStreamSynchronize(st_));
-    launches_per_prop_ = (use_sweep_ || use_sweep64_) ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
+    launches_per_prop_ = real_ ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
     launches_per_iter_ = launches_per_prop_ + 2 + 2 + (p.scft == 1 ? 4 : 1);
 }
 
@@ -494,9 +482,8 @@ ModelAB::~ModelAB() {
     if (gprop_) cudaGraphExecDestroy(gprop_);
     if (gpost_) cudaGraphExecDestroy(gpost_);
     delete chain_;
+    delete real_;
     if (axs_) cudaFree(axs_);
-    if (swbar_) cudaFree(swbar_);
-    if (swerr_) cudaFree(swerr_);
     if (st_) cudaStreamDestroy(st_);
 }
 
@@ -533,83 +520,13 @@ void ModelAB::set_fields(const double* wA, const double* wB, bool dev) {
     forward_done_ = false;
 }
 
-// The x-tile variant of the generic persistent sweep for this grid, timed
-// once per device and grid shape in a process (whole sweeps on this solve's
-// buffers, before its fields are set; the variants compute the same values,
-// so the choice only changes the time) and cached.  PS_B200_AUTOTUNE=0
-// keeps the default variant, PS_B200_SWEEP_VARIANT=v forces variant v.
-void ModelAB::tune_sweep() {
-    const char* force = getenv("PS_B200_SWEEP_VARIANT");
-    if (force && force[0] >= '0' && force[0] < '0' + kSweepVariants) {
-        sweep_variant_ = force[0] - '0';
-        return;
-    }
-    const char* at = getenv("PS_B200_AUTOTUNE");
-    if (at && at[0] == '0') return;
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, int, int>, int> cache;   // (device, Lx, Ly, Lz) -> variant
-    int dev = 0;
-    PS_CUDA(cudaGetDevice(&dev));
-    const auto key = std::make_tuple(dev, p_.Lx, p_.Ly, p_.Lz);
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
-        sweep_variant_ = it->second;
-        return;
-    }
-    // finite data for the timed sweeps (set_fields overwrites the factors)
-    for (double* f : {eFA_.p, eHA_.p, eFB_.p, eHB_.p}) launch_fill(f, M_, 1.0, st_);
-    const SweepArgs a = sweep_descriptor();
-    cudaEvent_t e0, e1;
-    PS_CUDA(cudaEventCreate(&e0));
-    PS_CUDA(cudaEventCreate(&e1));
-    double best = 1e30;
-    char line[512];
-    int n = std::snprintf(line, sizeof(line), "grid %dx%dx%d persistent sweep, x-tile columns (us per step):",
-                          p_.Lx, p_.Ly, p_.Lz);
-    for (int v = 0; v < kSweepVariants; v++) {
-        auto run = [&]() {
-            PS_CUDA(cudaMemsetAsync(swbar_, 0, 32 * sizeof(unsigned), st_));
-            sweep_launch(a, p_.Lx, p_.Ly, p_.Lz, sweep_grid_, 1, st_, v);
-        };
-        run();
-        PS_CUDA(cudaEventRecord(e0, st_));
-        for (int r = 0; r < 3; r++) run();
-        PS_CUDA(cudaEventRecord(e1, st_));
-        PS_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        PS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        const double us = 1e3 * ms / 3.0 / Ns_;
-        if (n > 0 && n < (int)sizeof(line))
-            n += std::snprintf(line + n, sizeof(line) - n, " %d=%.1f", sweep_xtile_columns(p_.Lx, p_.Ly, p_.Lz, v), us);
-        if (us < best) {
-            best = us;
-            sweep_variant_ = v;
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    int err = 0;
-    PS_CUDA(cudaMemcpy(&err, swerr_, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err) throw Error(-3, "persistent sweep reported an error while it was timed");
-    if (n > 0 && n < (int)sizeof(line))
-        std::snprintf(line + n, sizeof(line) - n, " -> %d\n", sweep_xtile_columns(p_.Lx, p_.Ly, p_.Lz, sweep_variant_));
-    tuning_note(line);
-    cache[key] = sweep_variant_;
-}
-
-SweepArgs ModelAB::sweep_descriptor() const {
-    if (!use_sweep_) throw Error(-2, "this solve has no generic persistent sweep");
-    SweepArgs a{};
-    a.hf = hf_.p; a.hc = hc_.p;
-    a.Z1 = swZ_.c(); a.Z2 = swZ_.c() + M_; a.Z3 = swZ_.c() + 2 * M_;
-    a.uf = swU_.p; a.uc = swU_.p + M_;
-    a.eFA = eFA_.p; a.eHA = eHA_.p; a.eFB = eFB_.p; a.eHB = eHB_.p;
-    a.L1 = swL1_.p; a.L2 = swL2_.p;
-    a.LA = LA_; a.LB = LB_; a.Ns = Ns_;
-    a.bar = swbar_; a.err = swerr_;
-    a.bstride_batch = 0; a.bstride_hist = 0; a.bstride_L = 0;
-    return a;
+RealProblem ModelAB::sweep_descriptor() const {
+    if (!real_) throw Error(-2, "this solve has no persistent sweep");
+    // forward chain: A then B; complementary chain: B then A
+    const int never = 1 << 30;
+    const RealLane lanes[2] = {{hf_.p, {eFA_.p, eFB_.p, eFB_.p}, {eHA_.p, eHB_.p, eHB_.p}, {LA_, never}},
+                               {hc_.p, {eFB_.p, eFA_.p, eFA_.p}, {eHB_.p, eHA_.p, eHA_.p}, {LB_, never}}};
+    return real_->problem(lanes, Ns_);
 }
 
 void ModelAB::enqueue_propagate() { enqueue_propagate(st_); }
@@ -617,21 +534,8 @@ void ModelAB::enqueue_propagate() { enqueue_propagate(st_); }
 void ModelAB::enqueue_propagate(cudaStream_t s) {
     // propagators: forward chain qA -> qB, complementary chain qBc -> qAc
     // (Model_AB.cc:139-145, 187-193)
-    if (use_sweep64_) {
-        SweepArgs a{};
-        a.hf = hf_.p; a.hc = hc_.p;
-        a.Z1 = swZ_.c(); a.Z2 = swZ_.c() + M_; a.Z3 = swZ_.c() + 2 * M_;
-        a.eFA = eFA_.p; a.eHA = eHA_.p; a.eFB = eFB_.p; a.eHB = eHB_.p;
-        a.LA = LA_; a.LB = LB_; a.Ns = Ns_;
-        a.bar = swbar_; a.err = swerr_;
-        PS_CUDA(cudaMemsetAsync(swbar_, 0, 64 * sizeof(unsigned), s));
-        sweep64_launch(a, swTab_.p, sweep_grid_, s);
-        return;
-    }
-    if (use_sweep_) {
-        const SweepArgs a = sweep_descriptor();
-        PS_CUDA(cudaMemsetAsync(swbar_, 0, 32 * sizeof(unsigned), s));
-        sweep_launch(a, p_.Lx, p_.Ly, p_.Lz, sweep_grid_, 1, s, sweep_variant_);
+    if (real_) {
+        real_->enqueue(sweep_descriptor(), s);
         return;
     }
     if (p_.mde == 2) {
@@ -800,12 +704,7 @@ int ModelAB::status() {
         PS_CUDA(cudaStreamSynchronize(st_));
         st |= s.status;
     }
-    if (swerr_) {
-        int e = 0;
-        PS_CUDA(cudaMemcpyAsync(&e, swerr_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
-        if (e) st |= 2;
-    }
+    if (real_ && real_->error(st_)) st |= 2;
     return st;
 }
 
@@ -857,6 +756,15 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
         }
         chain_->set_tables(L1, L2);
     }
+    // one chain of a 3D grid takes the persistent sweep (as Model_AB's do)
+    const char* force = getenv("PS_B200_LINE_PASSES");
+    if (!(force && force[0] == '1') && (scheme == SCHEME_RQM4 || (scheme == SCHEME_OS2 && cell_separable(cell_))) &&
+        real_sweep_supported(Lx, Ly, Lz)) {
+        const int n[3] = {Lx, Ly, Lz};
+        double k[3];
+        axis_k2(cell_, k);
+        real_ = new RealSweep(n, k, ds, 1, scheme == SCHEME_OS2);
+    }
     eF_.alloc(2 * M_);
     eH_.alloc(2 * M_);
     zero_.alloc(M_);
@@ -867,6 +775,7 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
 
 UpdaterCtx::~UpdaterCtx() {
     delete chain_;
+    delete real_;
     if (st_) cudaStreamDestroy(st_);
 }
 
@@ -885,6 +794,11 @@ void UpdaterCtx::solve_device(const double* w, double* qs, int len, cudaStream_t
     }
     // exp(-w ds/2), exp(-w ds/4) (RQM4.cc:49-52, PseudoSpectral.cc:234-235)
     launch_factors(w, w, M_, ds_, ds_, eF_.p, eH_.p, eF_.p + M_, eH_.p + M_, 1, 0, st);
+    if (real_) {
+        const RealLane lane{qs, {eF_.p, eF_.p, eF_.p}, {eH_.p, eH_.p, eH_.p}, {len, len}};
+        real_->enqueue(real_->problem(&lane, len - 1), st);
+        return;
+    }
     // lane c carries nothing: zero factors, zero input, scratch output
     LaneFactors lf{{eF_.p, eF_.p}, {eH_.p, eH_.p}, len};
     LaneFactors lc{{zero_.p, zero_.p}, {zero_.p, zero_.p}, len};
@@ -902,6 +816,7 @@ void UpdaterCtx::solve_host(const double* w, double* qs, int len) {
         PS_CUDA(cudaMemcpyAsync(qs + M_, dqs_.p + M_, sizeof(double) * (size_t)(len - 1) * M_,
                                 cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaStreamSynchronize(st_));
+    if (real_ && real_->error(st_)) throw Error(-3, "the propagator sweep reported a barrier timeout");
 }
 
 }  // namespace ps

@@ -7,6 +7,7 @@
 #include "ps_internal.h"
 #include "anderson.h"
 #include "sweep.h"
+#include "real_sweep.h"
 
 namespace ps {
 
@@ -35,6 +36,10 @@ void cell_init(Cell& c);   // throws on bad parameters
 
 // -k^2 on an orthogonal cell (UnitCell.cc:368-418)
 std::vector<double> k2_orthogonal(const Cell& c, int Lx, int Ly, int Lz);
+// -(wave number)^2 of index 1 along each axis of the orthogonal k2 table
+void axis_k2(const Cell& c, double k[3]);
+// whether |q|^2 of the general cell separates into one term an axis
+bool cell_separable(const Cell& c);
 // exp(-ds |q|^2), 27-image minimum (UnitCell.cc:321-359)
 std::vector<double> k_laplacian(const Cell& c, int Lx, int Ly, int Lz, double ds);
 
@@ -180,11 +185,10 @@ public:
     long iterations() const { return iter_; }
     int status();
     const ModelABParams& params() const { return p_; }
-    bool persistent_sweep() const { return use_sweep_; }       // generic sweep (sweep.cu)
-    bool persistent_sweep64() const { return use_sweep64_; }   // 64^3 sweep (sweep64.cu)
-    // the generic sweep's arguments for this solve (its own pointers, batch
-    // strides 0, its barrier words and error flag)
-    SweepArgs sweep_descriptor() const;
+    bool persistent_sweep() const { return real_ != nullptr; }   // real_sweep.cu
+    // the sweep's description of this solve (its own work fields, barrier
+    // words and error flag)
+    RealProblem sweep_descriptor() const;
     // the propagator sweeps of one iteration on stream s
     void enqueue_propagate(cudaStream_t s);
     // Adjoint of the forward map (wA, wB) -> (phiA, phiB, Q) at fixed fields:
@@ -217,7 +221,6 @@ private:
     void enqueue_post() { enqueue_post(st_); }
     void ensure_graphs();
     void init_anderson(const double* wA, const double* wB, bool device_ptrs);
-    void tune_sweep();
     void adjoint_weights(std::vector<double>& wAf, std::vector<double>& wBf) const;
     void ensure_adjoint_buffers(bool spec);
     ModelABParams p_;
@@ -226,14 +229,7 @@ private:
     double dsA_, dsB_;
     int ruleA_, ruleB_;
     PairChain* chain_ = nullptr;
-    // persistent sweep (RQM4 on the shapes sweep_supported() lists)
-    bool use_sweep_ = false;
-    bool use_sweep64_ = false;
-    int sweep_grid_ = 0;
-    int sweep_variant_ = 0;              // x-tile variant of the generic sweep (tune_sweep)
-    DevBuf swZ_, swU_, swL1_, swL2_, swTab_;
-    unsigned* swbar_ = nullptr;
-    int* swerr_ = nullptr;
+    RealSweep* real_ = nullptr;          // persistent sweep (3D grids, RQM4 and OS2)
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t gprop_ = nullptr, gpost_ = nullptr;
     DevBuf hf_, hc_, wA_, wB_, yita_, phiA_, phiB_, eFA_, eHA_, eFB_, eHB_;
@@ -292,12 +288,9 @@ public:
     void enqueue_propagate(cudaStream_t s);
     void enqueue_post(cudaStream_t s);
     int launches_post() const { return 2 + 3 + (p_.scft == 1 ? 4 : 1); }
-    // the generic persistent sweep (32^3, 48^3 grids; 64^3 where the 64^3
-    // sweep cannot run) with three factor sets
-    bool persistent_sweep() const { return use_sweep_; }
-    // the 64^3 sweep (sweep64.cu) with three factor sets
-    bool persistent_sweep64() const { return use_sweep64_; }
-    SweepArgs sweep_descriptor() const;
+    // the persistent sweep with three factor sets
+    bool persistent_sweep() const { return real_ != nullptr; }
+    RealProblem sweep_descriptor() const;
     const ModelABCParams& params() const { return p_; }
 
 private:
@@ -314,12 +307,7 @@ private:
     cudaGraphExec_t graph_ = nullptr;
     long iter_ = 0;
     bool fields_set_ = false;
-    bool use_sweep_ = false;
-    bool use_sweep64_ = false;
-    int sweep_grid_ = 0;
-    DevBuf swZ_, swU_, swL1_, swL2_, swTab_;
-    unsigned* swbar_ = nullptr;
-    int* swerr_ = nullptr;
+    RealSweep* real_ = nullptr;
 };
 
 // Single propagator updater behind the Updater C-ABI (RQM4 / OS2 / ETDRK4)
@@ -339,6 +327,7 @@ private:
     int etd_M_;
     long M_;
     PairChain* chain_ = nullptr;
+    RealSweep* real_ = nullptr;
     DevBuf eF_, eH_, zero_, scratch_, dw_, dqs_;
     cudaStream_t st_ = nullptr;
 };

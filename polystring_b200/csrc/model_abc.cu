@@ -66,35 +66,11 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
     }
     chain_->set_tables(L1, L2);
     const char* force = getenv("PS_B200_LINE_PASSES");
-    const char* generic = getenv("PS_B200_GENERIC_SWEEP");
-    const bool allow = !(force && force[0] == '1');
-    // 64^3 grids take the 64^3 sweep where its clusters fit (as Model_AB)
-    use_sweep64_ = allow && sweep64_supported(p.Lx, p.Ly, p.Lz) && !(generic && generic[0] == '1');
-    if (use_sweep64_) {
-        sweep_grid_ = sweep64_prepare();
-        use_sweep64_ = sweep_grid_ > 0;
-    }
-    use_sweep_ = allow && !use_sweep64_ && sweep_supported(p.Lx, p.Ly, p.Lz);
-    if (use_sweep64_) {
-        swZ_.alloc(6 * (size_t)M_);
-        const std::vector<double> tab = sweep64_axis_tables(p_.cell.l, ds_[0]);
-        swTab_.alloc(tab.size());
-        PS_CUDA(cudaMemcpy(swTab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMalloc(&swbar_, 64 * sizeof(unsigned)));
-        PS_CUDA(cudaMalloc(&swerr_, sizeof(int)));
-        PS_CUDA(cudaMemset(swerr_, 0, sizeof(int)));
-    }
-    if (use_sweep_) {
-        sweep_grid_ = sweep_prepare(p.Lx, p.Ly, p.Lz);
-        swZ_.alloc(6 * (size_t)M_);
-        swU_.alloc(2 * (size_t)M_);
-        swL1_.alloc(M_);
-        swL2_.alloc(M_);
-        PS_CUDA(cudaMemcpy(swL1_.p, L1.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMemcpy(swL2_.p, L2.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
-        PS_CUDA(cudaMalloc(&swbar_, 32 * sizeof(unsigned)));
-        PS_CUDA(cudaMalloc(&swerr_, sizeof(int)));
-        PS_CUDA(cudaMemset(swerr_, 0, sizeof(int)));
+    if (!(force && force[0] == '1') && real_sweep_supported(p.Lx, p.Ly, p.Lz)) {
+        const int n[3] = {p.Lx, p.Ly, p.Lz};
+        double k[3];
+        axis_k2(p_.cell, k);
+        real_ = new RealSweep(n, k, ds_[0], 2, false);
     }
     hf_.alloc((size_t)(Ns_ + 1) * M_);
     hc_.alloc((size_t)(Ns_ + 1) * M_);
@@ -116,16 +92,15 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
     launch_fill(hf_.p, M_, 1.0, st_);
     launch_fill(hc_.p, M_, 1.0, st_);
     launch_fill(yita_.p, M_, 0.0, st_);
-    if (!use_sweep_ && !use_sweep64_) chain_->autotune(st_);
+    if (!real_) chain_->autotune(st_);
     PS_CUDA(cudaStreamSynchronize(st_));
 }
 
 ModelABC::~ModelABC() {
     if (graph_) cudaGraphExecDestroy(graph_);
     delete chain_;
+    delete real_;
     if (axs_) cudaFree(axs_);
-    if (swbar_) cudaFree(swbar_);
-    if (swerr_) cudaFree(swerr_);
     if (st_) cudaStreamDestroy(st_);
 }
 
@@ -157,35 +132,18 @@ void ModelABC::set_fields(const double* const w[3], bool dev) {
     fields_set_ = true;
 }
 
-SweepArgs ModelABC::sweep_descriptor() const {
-    if (!use_sweep_) throw Error(-2, "this solve has no generic persistent sweep");
-    SweepArgs a{};
-    a.hf = hf_.p; a.hc = hc_.p;
-    a.Z1 = swZ_.c(); a.Z2 = swZ_.c() + M_; a.Z3 = swZ_.c() + 2 * M_;
-    a.uf = swU_.p; a.uc = swU_.p + M_;
-    a.eFA = eF_[0].p; a.eHA = eH_[0].p; a.eFB = eF_[1].p; a.eHB = eH_[1].p; a.eFC = eF_[2].p; a.eHC = eH_[2].p;
-    a.L1 = swL1_.p; a.L2 = swL2_.p;
-    a.LA = L_[0]; a.LB = L_[1]; a.LC = L_[2]; a.Ns = Ns_;
-    a.bar = swbar_; a.err = swerr_;
-    return a;
+RealProblem ModelABC::sweep_descriptor() const {
+    if (!real_) throw Error(-2, "this solve has no persistent sweep");
+    // forward chain: A, B, C; complementary chain: C, B, A
+    const RealLane lanes[2] = {
+        {hf_.p, {eF_[0].p, eF_[1].p, eF_[2].p}, {eH_[0].p, eH_[1].p, eH_[2].p}, {L_[0], L_[0] + L_[1]}},
+        {hc_.p, {eF_[2].p, eF_[1].p, eF_[0].p}, {eH_[2].p, eH_[1].p, eH_[0].p}, {L_[2], L_[2] + L_[1]}}};
+    return real_->problem(lanes, Ns_);
 }
 
 void ModelABC::enqueue_propagate(cudaStream_t s) {
-    if (use_sweep64_) {
-        SweepArgs a{};
-        a.hf = hf_.p; a.hc = hc_.p;
-        a.Z1 = swZ_.c(); a.Z2 = swZ_.c() + M_; a.Z3 = swZ_.c() + 2 * M_;
-        a.eFA = eF_[0].p; a.eHA = eH_[0].p; a.eFB = eF_[1].p; a.eHB = eH_[1].p; a.eFC = eF_[2].p; a.eHC = eH_[2].p;
-        a.LA = L_[0]; a.LB = L_[1]; a.LC = L_[2]; a.Ns = Ns_;
-        a.bar = swbar_; a.err = swerr_;
-        PS_CUDA(cudaMemsetAsync(swbar_, 0, 64 * sizeof(unsigned), s));
-        sweep64_launch(a, swTab_.p, sweep_grid_, s);
-        return;
-    }
-    if (use_sweep_) {
-        const SweepArgs a = sweep_descriptor();
-        PS_CUDA(cudaMemsetAsync(swbar_, 0, 32 * sizeof(unsigned), s));
-        sweep_launch(a, p_.Lx, p_.Ly, p_.Lz, sweep_grid_, 1, s, sweep_default_variant(p_.Lx, p_.Ly, p_.Lz));
+    if (real_) {
+        real_->enqueue(sweep_descriptor(), s);
         return;
     }
     // lane f: A for t < LA, B up to LA + LB, then C; lane c: C, B, A
@@ -328,12 +286,7 @@ int ModelABC::status() {
         PS_CUDA(cudaStreamSynchronize(st_));
         st |= s.status;
     }
-    if (swerr_) {
-        int e = 0;
-        PS_CUDA(cudaMemcpyAsync(&e, swerr_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
-        if (e) st |= 2;
-    }
+    if (real_ && real_->error(st_)) st |= 2;
     return st;
 }
 

@@ -1,0 +1,85 @@
+// real_sweep.h -- propagator sweeps built on real line operators
+// (real_line.cuh): 3D grids in real_sweep.cu.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "ps_internal.h"
+
+namespace ps {
+
+// One chain of a solve: its history ((Ns + 1) slices, slice 0 the head) and
+// the Boltzmann factors e^{-w ds/2}, e^{-w ds/4} of the blocks it runs through,
+// block 0 before step sw[0], block 1 before sw[1], then block 2.
+struct RealLane {
+    double* hist;
+    const double* eF[3];
+    const double* eH[3];
+    int sw[2];
+};
+
+// One solve of a sweep: nl chains (one or two) of Ns contour steps.
+struct RealProblem {
+    RealLane lane[2];
+    double *W, *Z;        // work fields, nl x M each
+    const double* frag;   // B fragments of the axes' operators (full step, half step)
+    int fo[3], nfrag;     // where each axis's start (axes of equal length and spacing share), doubles in all
+    unsigned* bar;        // barrier counters (one a chain, 16 words apart), zeroed before the launch
+    int* err;             // nonzero after a barrier timeout
+    int Lx, Ly, Lz, Ns, nl;
+    int os2;              // second-order splitting: full steps only
+    int xcols;            // columns of an x-pass task (a multiple of 8)
+    int rkeep, xkeep;     // factors kept in shared memory: of the rows, of that many x-pass tasks a warp
+    int cta0, ncta;       // the solve's first CTA in a shared launch, CTAs of each chain
+};
+
+// the axes' operators of an orthogonal cell, exp(h k r^2) per axis for h = ds and
+// ds / 2, k = -(wave number)^2 at index 1; fo[a]: where axis a's start (axes
+// of the same length and k share theirs)
+std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, int fo[3]);
+
+// whether a 3D grid has this sweep
+bool real_sweep_supported(int Lx, int Ly, int Lz);
+// sets kernel attributes; returns the CTAs of one solve alone (one an SM), or
+// with `shared` those that a shared launch can have resident at once, with nfrag
+// doubles of fragments
+int real_sweep_prepare(int Lx, int Ly, int Lz, int nfrag, bool shared);
+// CTAs one chain can keep busy
+int real_sweep_tasks(int Lx, int Ly, int Lz);
+// time of a contour step with `per` CTAs a chain, in units of a shared-launch cost model
+double real_sweep_step_cost(int Lx, int Ly, int Lz, int per);
+// x-tile variants (columns a task; same arithmetic)
+constexpr int kRealVariants = 3;
+int real_sweep_columns(int variant);
+// ncta CTAs a chain
+void real_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
+// n solves of one shape described in device memory, grid CTAs in all, nfrag the
+// largest of the solves'
+void real_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int Lz, int nfrag, int grid, cudaStream_t st);
+
+// The work fields, operators and barrier words of one solve's sweep.
+class RealSweep {
+public:
+    // k: -(wave number)^2 of index 1 along each axis; nl chains
+    RealSweep(const int n[3], const double k[3], double ds, int nl, bool os2);
+    ~RealSweep();
+    RealSweep(const RealSweep&) = delete;
+    RealSweep& operator=(const RealSweep&) = delete;
+    // the solve's description: chains and number of steps
+    RealProblem problem(const RealLane* lanes, int Ns) const;
+    // chooses the x-tile variant by timing whole sweeps of p, once per device
+    // and grid shape in a process (PS_B200_AUTOTUNE=0 keeps the default,
+    // PS_B200_SWEEP_VARIANT=v forces variant v)
+    void tune(const RealProblem& p, cudaStream_t st);
+    void enqueue(const RealProblem& p, cudaStream_t st) const;
+    int error(cudaStream_t st) const;   // barrier error flag (synchronises)
+
+private:
+    int n_[3], nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
+    double *work_ = nullptr, *frag_ = nullptr;
+    unsigned* bar_ = nullptr;   // 32 words, then the error flag
+};
+
+}  // namespace ps

@@ -281,7 +281,7 @@ void StringAB::enqueue_scft_iteration() {
         a.eFA = eFA_.p; a.eHA = eHA_.p; a.eFB = eFB_.p; a.eHB = eHB_.p;
         a.ktab = clK_.p;
         a.LA = LA_; a.LB = LB_; a.Ns = Ns_;
-        a.bstride_batch = M_; a.bstride_hist = hstride; a.bstride_L = 0;
+        a.bstride_batch = M_; a.bstride_hist = hstride;
         cluster_sweep_launch(a, p_.Lx, p_.Ly, p_.Lz, nloc_, st_);
     } else {
         LaneFactors lf{{eFA_.p, eFB_.p}, {eHA_.p, eHB_.p}, LA_};
