@@ -141,6 +141,30 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
         };
         int nfrag = 0;
         for (int k : kv.second) nfrag = std::max(nfrag, descriptor(k).nfrag);
+        auto emplace = [&](int i0, int n, int per, const std::vector<int>& ks) {
+            chunks_.emplace_back();
+            SweepChunk& c = chunks_.back();
+            c.Lx = Lx; c.Ly = Ly; c.Lz = Lz; c.nfrag = nfrag;
+            c.n = n;
+            c.per = per;
+            PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * (size_t)n));
+            std::vector<RealProblem> d(n);
+            for (int i = 0; i < n; i++) {
+                d[i] = descriptor(ks[i0 + i]);
+                d[i].bar = c.bar + 32 * (size_t)i;
+                d[i].cta0 = 2 * i * per;
+                d[i].ncta = per;
+            }
+            PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
+            PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+        };
+        if (Lz == 1) {
+            // 2D solves: a CTA a chain, independent of each other, longest first
+            std::vector<int> ks = kv.second;
+            std::stable_sort(ks.begin(), ks.end(), [&](int a, int b) { return Ns_of(a) > Ns_of(b); });
+            emplace(0, (int)ks.size(), 0, ks);
+            continue;
+        }
         const int resident = real_sweep_prepare(Lx, Ly, Lz, nfrag, true);
         const int tasks = real_sweep_tasks(Lx, Ly, Lz);
         // A launch of n solves gives each per = resident / n CTAs (at most the
@@ -165,22 +189,8 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
         for (int i = nk; i > 0; i = from[i]) runs.push_back({from[i], i});
         std::reverse(runs.begin(), runs.end());
         for (const auto& run : runs) {
-            const size_t i0 = (size_t)run.first;
-            chunks_.emplace_back();
-            SweepChunk& c = chunks_.back();
-            c.Lx = Lx; c.Ly = Ly; c.Lz = Lz; c.nfrag = nfrag;
-            c.n = run.second - run.first;
-            c.per = per_of(c.n);
-            PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * (size_t)c.n));
-            std::vector<RealProblem> d(c.n);
-            for (int i = 0; i < c.n; i++) {
-                d[i] = descriptor(ks[i0 + i]);
-                d[i].bar = c.bar + 32 * (size_t)i;
-                d[i].cta0 = 2 * i * c.per;
-                d[i].ncta = c.per;
-            }
-            PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
-            PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+            const int n = run.second - run.first;
+            emplace(run.first, n, per_of(n), ks);
         }
     }
 }
@@ -260,8 +270,12 @@ void BatchAB::build_group(Group& g) {
 void BatchAB::enqueue_iteration() {
     int launches = 0;
     for (const SweepChunk& c : chunks_) {
-        PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-        real_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.Lz, c.nfrag, 2 * c.per * c.n, st_);
+        if (c.Lz == 1) {
+            plane_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.nfrag, st_);
+        } else {
+            PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
+            real_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.Lz, c.nfrag, 2 * c.per * c.n, st_);
+        }
         launches++;
     }
     int Ns_max = 0;

@@ -601,7 +601,7 @@ void cluster_launch_t(SweepArgs a, int nbatch, cudaStream_t st) {
 }  // namespace
 
 // (LX, LY, CTAs per cluster)
-#define PS_CLUSTER_SHAPES(X) X(32, 32, 4) X(64, 64, 4) X(128, 128, 8)
+#define PS_CLUSTER_SHAPES(X) X(128, 128, 8)
 
 bool cluster_sweep_supported(int Lx, int Ly, int Lz) {
 #define PS_X(x, y, c) if (Lx == x && Ly == y && Lz == 1) return true;

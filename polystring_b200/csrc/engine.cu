@@ -436,11 +436,12 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
         }
         chain_->set_tables(L1, L2);
     }
-    // 3D grids of orthogonal cells propagate by the persistent sweep on real
-    // line operators (PS_B200_LINE_PASSES=1 keeps the line passes)
+    // the chains run in persistent sweeps on real line operators where the
+    // diffusion step separates into axes and the grid has one
+    // (PS_B200_LINE_PASSES=1 keeps the line passes)
     const char* force = getenv("PS_B200_LINE_PASSES");
     if (!(force && force[0] == '1') && (p.mde == 0 || (p.mde == 1 && cell_separable(p_.cell))) &&
-        real_sweep_supported(p.Lx, p.Ly, p.Lz)) {
+        RealSweep::supported(p.Lx, p.Ly, p.Lz)) {
         const int n[3] = {p.Lx, p.Ly, p.Lz};
         double k[3];
         axis_k2(p_.cell, k);
@@ -467,7 +468,8 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     launch_fill(hf_.p, M_, 1.0, st_);
     launch_fill(hc_.p, M_, 1.0, st_);
     launch_fill(yita_.p, M_, 0.0, st_);
-    if (!real_ && !batch_member) chain_->autotune(st_);
+    // (2D grids: the adjoint runs the line passes)
+    if ((!real_ || p.dim == 2) && !batch_member) chain_->autotune(st_);
     if (real_ && !batch_member) {
         // finite data for the timed sweeps (set_fields overwrites the factors)
         for (double* f : {eFA_.p, eHA_.p, eFB_.p, eHB_.p}) launch_fill(f, M_, 1.0, st_);
@@ -756,10 +758,10 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
         }
         chain_->set_tables(L1, L2);
     }
-    // one chain of a 3D grid takes the persistent sweep (as Model_AB's do)
+    // one chain takes the persistent sweep as Model_AB's two do
     const char* force = getenv("PS_B200_LINE_PASSES");
     if (!(force && force[0] == '1') && (scheme == SCHEME_RQM4 || (scheme == SCHEME_OS2 && cell_separable(cell_))) &&
-        real_sweep_supported(Lx, Ly, Lz)) {
+        RealSweep::supported(Lx, Ly, Lz)) {
         const int n[3] = {Lx, Ly, Lz};
         double k[3];
         axis_k2(cell_, k);

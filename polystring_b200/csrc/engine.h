@@ -6,7 +6,6 @@
 
 #include "ps_internal.h"
 #include "anderson.h"
-#include "sweep.h"
 #include "real_sweep.h"
 
 namespace ps {

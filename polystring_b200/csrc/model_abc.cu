@@ -66,7 +66,7 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
     }
     chain_->set_tables(L1, L2);
     const char* force = getenv("PS_B200_LINE_PASSES");
-    if (!(force && force[0] == '1') && real_sweep_supported(p.Lx, p.Ly, p.Lz)) {
+    if (!(force && force[0] == '1') && RealSweep::supported(p.Lx, p.Ly, p.Lz)) {
         const int n[3] = {p.Lx, p.Ly, p.Lz};
         double k[3];
         axis_k2(p_.cell, k);

@@ -135,6 +135,11 @@ struct RealLine {
     // the operator's table; lanes read consecutive doubles around one entry.
     __device__ __forceinline__ static void apply_parts(double (&x)[E], const double* th) {
         const int lane = threadIdx.x & 31, og = real_column_orbit(lane >> 2), j = lane & 3;
+        if constexpr (!WHOLE) {
+            // the parts go on past the last orbit: what the lane holds there counts as zero
+#pragma unroll
+            for (int b = 0; b < 4; b++) x[4 * (S - 1) + b] = j + 4 * (S - 1) < O ? x[4 * (S - 1) + b] : 0.0;
+        }
         fold(x);
 #pragma unroll
         for (int h = 0; h < 2; h++) {

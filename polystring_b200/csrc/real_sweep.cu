@@ -444,10 +444,11 @@ void launch(const RealProblem& p, const RealProblem* d, int n, size_t smem, bool
 
 }  // namespace
 
-std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, int fo[3]) {
+std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, bool parts, int fo[3]) {
     std::vector<double> out;
     for (int a = 0; a < 3; a++) {
         fo[a] = -1;
+        if (n[a] == 1) continue;
         for (int b = 0; b < a; b++)
             if (n[b] == n[a] && k[b] == k[a]) fo[a] = fo[b];
         if (fo[a] >= 0) continue;
@@ -458,7 +459,8 @@ std::vector<double> real_operator_tables(const int n[3], const double k[3], doub
                 const int r = i < n[a] / 2 + 1 ? i : n[a] - i;
                 L[i] = exp(h * (k[a] * r * r));
             }
-            real_fragments(n[a], L, out);
+            if (parts) real_parts(n[a], L, out);
+            else real_fragments(n[a], L, out);
         }
     }
     return out;
@@ -523,14 +525,27 @@ void real_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int Lz,
 // ---------------------------------------------------------------------------
 // RealSweep
 // ---------------------------------------------------------------------------
+bool RealSweep::supported(int Lx, int Ly, int Lz) {
+    if (Ly == 1 && Lz == 1) return line_sweep_supported(Lx);
+    if (Lz == 1) return plane_sweep_supported(Lx, Ly);
+    return real_sweep_supported(Lx, Ly, Lz);
+}
+
 RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool os2) : nl_(nl), os2_(os2) {
     std::copy(n, n + 3, n_);
+    dim_ = n[2] > 1 ? 3 : n[1] > 1 ? 2 : 1;
     const size_t M = (size_t)n[0] * n[1] * n[2];
     variant_ = 0;
-    const std::vector<double> f = real_operator_tables(n, k, ds, fo_);
+    ncta_ = 0;
+    const std::vector<double> f = real_operator_tables(n, k, ds, dim_ == 1, fo_);
     nfrag_ = (int)f.size();
-    ncta_ = std::max(1, std::min(real_sweep_prepare(n[0], n[1], n[2], nfrag_, false) / nl, real_sweep_tasks(n[0], n[1], n[2])));
-    PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
+    if (dim_ == 3) {
+        ncta_ = std::max(1, std::min(real_sweep_prepare(n[0], n[1], n[2], nfrag_, false) / nl,
+                                     real_sweep_tasks(n[0], n[1], n[2])));
+        PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
+    } else if (dim_ == 2) {
+        plane_sweep_prepare();
+    }
     PS_CUDA(cudaMalloc(&frag_, sizeof(double) * f.size()));
     PS_CUDA(cudaMemcpy(frag_, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
     PS_CUDA(cudaMalloc(&bar_, 33 * sizeof(unsigned)));
@@ -563,6 +578,8 @@ RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
 }
 
 void RealSweep::enqueue(const RealProblem& p, cudaStream_t st) const {
+    if (dim_ == 1) return line_sweep_launch(p, st);
+    if (dim_ == 2) return plane_sweep_launch(p, st);
     PS_CUDA(cudaMemsetAsync(bar_, 0, 32 * sizeof(unsigned), st));
     real_sweep_launch(p, ncta_, st);
 }
@@ -575,6 +592,7 @@ int RealSweep::error(cudaStream_t st) const {
 }
 
 void RealSweep::tune(const RealProblem& p0, cudaStream_t st) {
+    if (dim_ < 3) return;
     const char* force = getenv("PS_B200_SWEEP_VARIANT");
     if (force && force[0] >= '0' && force[0] < '0' + kRealVariants) {
         variant_ = force[0] - '0';

@@ -1,5 +1,5 @@
 // real_sweep.h -- propagator sweeps built on real line operators
-// (real_line.cuh): 3D grids in real_sweep.cu.
+// (real_line.cuh): 3D grids in real_sweep.cu, 1D and 2D grids in plane_sweep.cu.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -24,7 +24,7 @@ struct RealLane {
 struct RealProblem {
     RealLane lane[2];
     double *W, *Z;        // work fields, nl x M each
-    const double* frag;   // B fragments of the axes' operators (full step, half step)
+    const double* frag;   // the axes' operators (full step, half step): B fragments (2D, 3D) or parts (1D)
     int fo[3], nfrag;     // where each axis's start (axes of equal length and spacing share), doubles in all
     unsigned* bar;        // barrier counters (one a chain, 16 words apart), zeroed before the launch
     int* err;             // nonzero after a barrier timeout
@@ -38,7 +38,7 @@ struct RealProblem {
 // the axes' operators of an orthogonal cell, exp(h k r^2) per axis for h = ds and
 // ds / 2, k = -(wave number)^2 at index 1; fo[a]: where axis a's start (axes
 // of the same length and k share theirs)
-std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, int fo[3]);
+std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, bool parts, int fo[3]);
 
 // whether a 3D grid has this sweep
 bool real_sweep_supported(int Lx, int Ly, int Lz);
@@ -59,6 +59,16 @@ void real_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
 // largest of the solves'
 void real_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int Lz, int nfrag, int grid, cudaStream_t st);
 
+// 2D grids of up to 64 x 64 points, one CTA a chain
+bool plane_sweep_supported(int Lx, int Ly);
+void plane_sweep_prepare();
+void plane_sweep_launch(const RealProblem& p, cudaStream_t st);
+// n solves of two chains and one shape described in device memory
+void plane_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int nfrag, cudaStream_t st);
+// 1D grids
+bool line_sweep_supported(int Lx);
+void line_sweep_launch(const RealProblem& p, cudaStream_t st);
+
 // The work fields, operators and barrier words of one solve's sweep.
 class RealSweep {
 public:
@@ -67,6 +77,8 @@ public:
     ~RealSweep();
     RealSweep(const RealSweep&) = delete;
     RealSweep& operator=(const RealSweep&) = delete;
+    // whether a grid has a sweep
+    static bool supported(int Lx, int Ly, int Lz);
     // the solve's description: chains and number of steps
     RealProblem problem(const RealLane* lanes, int Ns) const;
     // chooses the x-tile variant by timing whole sweeps of p, once per device
@@ -74,10 +86,11 @@ public:
     // PS_B200_SWEEP_VARIANT=v forces variant v)
     void tune(const RealProblem& p, cudaStream_t st);
     void enqueue(const RealProblem& p, cudaStream_t st) const;
+    int fragments() const { return nfrag_; }   // doubles of the operators
     int error(cudaStream_t st) const;   // barrier error flag (synchronises)
 
 private:
-    int n_[3], nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
+    int n_[3], dim_, nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
     double *work_ = nullptr, *frag_ = nullptr;
     unsigned* bar_ = nullptr;   // 32 words, then the error flag
 };

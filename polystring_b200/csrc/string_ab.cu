@@ -193,6 +193,18 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
     if (p.mde != 0 && p.mde != 1) throw Error(-2, "string images use RQM4 or OS2");
     PS_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
     chain_ = new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : SCHEME_RQM4, nloc_);
+    // every image's chains in one launch of a persistent sweep per SCFT iteration
+    // where the 2D grid has one (PS_B200_LINE_PASSES=1 keeps the batched line
+    // passes)
+    const char* force = getenv("PS_B200_LINE_PASSES");
+    const bool lines = force && force[0] == '1';
+    if (!lines && p.Ly > 1 && p.Lz == 1 && (p.mde == 0 || cell_separable(p_.cell)) &&
+        plane_sweep_supported(p.Lx, p.Ly)) {
+        const int n[3] = {p.Lx, p.Ly, 1};
+        double k[3];
+        axis_k2(p_.cell, k);
+        real_ = new RealSweep(n, k, dsA_, 2, p.mde == 1);
+    }
     if (p.mde == 1) {
         chain_->set_tables(k_laplacian(p_.cell, p.Lx, p.Ly, p.Lz, dsA_), {});
     } else {
@@ -203,11 +215,9 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
             L2[i] = exp(0.5 * dsA_ * k2[i]);
         }
         chain_->set_tables(L1, L2);
-        // every image's propagators in one cluster-resident sweep per SCFT
-        // iteration where the 2D grid has one (PS_B200_LINE_PASSES=1 keeps
-        // the batched line passes)
-        const char* force = getenv("PS_B200_LINE_PASSES");
-        if (cluster_sweep_supported(p.Lx, p.Ly, p.Lz) && !(force && force[0] == '1')) {
+        // 128^2: every image's propagators in one cluster-resident sweep per
+        // SCFT iteration
+        if (!lines && cluster_sweep_supported(p.Lx, p.Ly, p.Lz)) {
             use_cluster_ = true;
             cluster_sweep_prepare(p.Lx, p.Ly, p.Lz, nloc_);
             // per-axis factors exp(h k_x^2), exp(h k_y^2) for h = ds, ds/2: the
@@ -221,13 +231,26 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
             PS_CUDA(cudaMemcpy(clK_.p, kt.data(), sizeof(double) * kt.size(), cudaMemcpyHostToDevice));
         }
     }
-    if (!use_cluster_) chain_->autotune(st_);
+    if (!use_cluster_ && !real_) chain_->autotune(st_);
     const size_t mM = (size_t)m * M_, nM = (size_t)nloc_ * M_;
     hf_.alloc((size_t)(Ns_ + 1) * nM);
     hc_.alloc((size_t)(Ns_ + 1) * nM);
     wa_.alloc(mM); wb_.alloc(mM); phiA_.alloc(mM); phiB_.alloc(mM);
     yita_.alloc(nM); eFA_.alloc(nM); eHA_.alloc(nM); eFB_.alloc(nM); eHB_.alloc(nM);
     ends_.alloc(4 * (size_t)M_);
+    if (real_) {
+        const int never = 1 << 30;
+        std::vector<RealProblem> d;
+        for (int b = 0; b < nloc_; b++) {
+            double *hf = hf_.p + (size_t)b * (Ns_ + 1) * M_, *hc = hc_.p + (size_t)b * (Ns_ + 1) * M_;
+            const double *fA = eFA_.p + b * M_, *hA = eHA_.p + b * M_, *fB = eFB_.p + b * M_, *hB = eHB_.p + b * M_;
+            const RealLane lanes[2] = {{hf, {fA, fB, fB}, {hA, hB, hB}, {LA_, never}},
+                                       {hc, {fB, fA, fA}, {hB, hA, hA}, {LB_, never}}};
+            d.push_back(real_->problem(lanes, Ns_));
+        }
+        PS_CUDA(cudaMalloc(&images_, sizeof(RealProblem) * d.size()));
+        PS_CUDA(cudaMemcpy(images_, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+    }
     cA_.alloc(cA.size()); cB_.alloc(cB.size());
     PS_CUDA(cudaMemcpy(cA_.p, cA.data(), sizeof(double) * cA.size(), cudaMemcpyHostToDevice));
     PS_CUDA(cudaMemcpy(cB_.p, cB.data(), sizeof(double) * cB.size(), cudaMemcpyHostToDevice));
@@ -250,6 +273,8 @@ StringAB::~StringAB() {
     if (grelax_) cudaGraphExecDestroy(grelax_);
     if (grepar_) cudaGraphExecDestroy(grepar_);
     delete chain_;
+    delete real_;
+    cudaFree(images_);
     if (st_) cudaStreamDestroy(st_);
 }
 
@@ -275,7 +300,9 @@ void StringAB::enqueue_scft_iteration() {
     const long off = (long)lo_ * M_;
     double *wa = wa_.p + off, *wb = wb_.p + off, *phiA = phiA_.p + off, *phiB = phiB_.p + off;
     double* scal = scal_.p + 8 * lo_;
-    if (use_cluster_) {
+    if (real_) {
+        plane_sweep_launch_many(images_, nloc_, p_.Lx, p_.Ly, real_->fragments(), st_);
+    } else if (use_cluster_) {
         SweepArgs a{};
         a.hf = hf_.p; a.hc = hc_.p;
         a.eFA = eFA_.p; a.eHA = eHA_.p; a.eFB = eFB_.p; a.eHB = eHB_.p;
@@ -431,7 +458,7 @@ void StringAB::get(int which, double* out, bool dev) {
 }
 
 int StringAB::launches_per_iteration() const {
-    const int prop = use_cluster_ ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
+    const int prop = real_ || use_cluster_ ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
     const int scft = prop + 2 + 2 + 1;
     return 2 + max_iter_ * scft + 2 + 2 + 1 + 2;
 }

@@ -30,7 +30,7 @@ public:
     long M() const { return M_; }
     int Ns() const { return Ns_; }
     int launches_per_iteration() const;
-    bool cluster_sweep() const { return use_cluster_; }
+    bool cluster_sweep() const { return use_cluster_ || real_; }
     cudaStream_t stream() const { return st_; }
 
 private:
@@ -49,7 +49,9 @@ private:
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t giter_ = nullptr, grelax_ = nullptr, grepar_ = nullptr;
     DevBuf hf_, hc_, wa_, wb_, yita_, phiA_, phiB_, eFA_, eHA_, eFB_, eHB_, ends_, cA_, cB_, scal_, S_, partial_;
-    // one thread-block cluster per image for the propagators (2D grids that have one)
+    RealSweep* real_ = nullptr;          // one CTA a chain (plane_sweep.cu): operators, and
+    RealProblem* images_ = nullptr;      // the images' descriptions on the device
+    // one thread-block cluster per image for the propagators (cluster_sweep.cu)
     bool use_cluster_ = false;
     DevBuf clK_;                         // per-axis exp(h k^2): x, y for h = ds, then ds / 2
     long iters_ = 0;
