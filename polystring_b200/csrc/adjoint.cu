@@ -225,10 +225,7 @@ void ModelAB::forward_only() {
     if (!fields_set_) throw Error(-6, "fields are not set");
     ensure_graphs();
     PS_CUDA(cudaGraphLaunch(gprop_, st_));
-    double* dQ = scal_.p + 0;
-    launch_mean(hf_.p + (long)Ns_ * M_, M_, partial_.p, dQ, st_);
-    launch_density(hf_.p, hc_.p + (long)LB_ * M_, LA_, M_, cA_.p, dsA_, dQ, 0.0, phiA_.p, 1, 0, 0, nullptr, st_);
-    launch_density(hf_.p + (long)LA_ * M_, hc_.p, LB_, M_, cB_.p, dsB_, dQ, 0.0, phiB_.p, 1, 0, 0, nullptr, st_);
+    enqueue_densities(st_);
     forward_done_ = true;
 }
 
@@ -260,6 +257,7 @@ void ModelAB::grad_w(const double* phiA_bar, const double* phiB_bar, double Q_ba
     if (!fields_set_) throw Error(-6, "fields are not set");
     if (p_.mde != 0) throw Error(-2, "the adjoint is provided for RQM4");
     ensure_adjoint_buffers(false);
+    if (sweep_adjoint(true)) return grad_w_sweep(phiA_bar, phiB_bar, Q_bar, gA, gB);
     forward_only();
     // pbar = phi_bar / Q; Qbar_total = Q_bar - (1/Q) sum(phi_bar phi)
     PS_CUDA(cudaMemcpyAsync(pbA_.p, phiA_bar, sizeof(double) * M_, cudaMemcpyHostToDevice, st_));
@@ -315,6 +313,7 @@ void ModelAB::grad_w(const double* phiA_bar, const double* phiB_bar, double Q_ba
 void ModelAB::stress(double* dFdl) {
     if (!fields_set_) throw Error(-6, "fields are not set");
     if (p_.mde != 0) throw Error(-2, "the adjoint is provided for RQM4");
+    if (sweep_adjoint(false)) return stress_sweep(dFdl);
     ensure_adjoint_buffers(true);
     forward_only();
     PS_CUDA(cudaMemsetAsync(gA_.p, 0, sizeof(double) * M_, st_));
@@ -357,6 +356,7 @@ void ModelAB::stress_checkpointed(int k, double* dFdl) {
     if (k > Ns_) k = Ns_;
     const int nseg = (Ns_ + k - 1) / k;
     ensure_adjoint_buffers(true);
+    if (real_) chain_->autotune(st_);   // models without a sweep did when they were made
     ck_.alloc((size_t)nseg * M_);
     seg_.alloc((size_t)(k + 1) * M_);
     if (zero_.n == 0) {

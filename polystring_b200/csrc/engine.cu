@@ -468,8 +468,7 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     launch_fill(hf_.p, M_, 1.0, st_);
     launch_fill(hc_.p, M_, 1.0, st_);
     launch_fill(yita_.p, M_, 0.0, st_);
-    // (2D grids: the adjoint runs the line passes)
-    if ((!real_ || p.dim == 2) && !batch_member) chain_->autotune(st_);
+    if (!real_ && !batch_member) chain_->autotune(st_);
     if (real_ && !batch_member) {
         // finite data for the timed sweeps (set_fields overwrites the factors)
         for (double* f : {eFA_.p, eHA_.p, eFB_.p, eHB_.p}) launch_fill(f, M_, 1.0, st_);
@@ -552,13 +551,17 @@ void ModelAB::enqueue_propagate(cudaStream_t s) {
     chain_->enqueue(hf_.p, hc_.p, 0, Ns_, lf, lc, 0, s);
 }
 
-void ModelAB::enqueue_post(cudaStream_t st) {
+void ModelAB::enqueue_densities(cudaStream_t st) {
     // Q = qB->Qt() (Model_AB.cc:195, Propagator.cc:85-93)
     double* dQ = scal_.p + 0;
     launch_mean(hf_.p + (long)Ns_ * M_, M_, partial_.p, dQ, st);
     // phiA = (1/Q) dsA sum c_s qA[s] qAc[LA - s]; phiB likewise (Model_AB.cc:196-199)
     launch_density(hf_.p, hc_.p + (long)LB_ * M_, LA_, M_, cA_.p, dsA_, dQ, 0.0, phiA_.p, 1, 0, 0, nullptr, st);
     launch_density(hf_.p + (long)LA_ * M_, hc_.p, LB_, M_, cB_.p, dsB_, dQ, 0.0, phiB_.p, 1, 0, 0, nullptr, st);
+}
+
+void ModelAB::enqueue_post(cudaStream_t st) {
+    enqueue_densities(st);
     if (p_.scft == 1) {
         AXArgs a{};
         a.state = axs_; a.n = p_.n_anderson; a.M = M_;

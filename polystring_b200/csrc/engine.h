@@ -222,6 +222,12 @@ private:
     void init_anderson(const double* wA, const double* wB, bool device_ptrs);
     void adjoint_weights(std::vector<double>& wAf, std::vector<double>& wBf) const;
     void ensure_adjoint_buffers(bool spec);
+    // the adjoint on the persistent sweeps (adjoint_sweep.cu)
+    bool sweep_adjoint(bool grad);
+    void forward_kept();
+    void grad_w_sweep(const double* phiA_bar, const double* phiB_bar, double Q_bar, double* gA, double* gB);
+    void stress_sweep(double* dFdl);
+    void enqueue_densities(cudaStream_t s);   // Q, phiA, phiB of the propagated chains
     ModelABParams p_;
     long M_;
     int LA_, LB_, Ns_;
@@ -238,6 +244,11 @@ private:
     AXState* axs_ = nullptr;
     DevBuf lam_, gA_, gB_, pbA_, pbB_, spec_, stress_part_;
     DevBuf ck_, seg_, zero_, scratch_;   // checkpointed stress
+    // kept fields of every step (half, full: forward chain, complementary
+    // chain), the same of the adjoint chains and their slices
+    DevBuf kept_[4], lkept_[4], lamh_[2];
+    DevBuf srcw_, chunks_, gpart_, sfrag_, spart_;
+    int adj_chunks_ = 0, sfo_[3] = {0, 0, 0};
     long iter_ = 0;
     bool fields_set_ = false;
     bool forward_done_ = false;   // Q, phi of the current fields are valid (forward_only)

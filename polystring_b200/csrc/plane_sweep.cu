@@ -111,6 +111,10 @@ __device__ __forceinline__ void columns(const Chain& c, int t) {
         double f[R::E];
         load_factors<N>(f, c.L->eF[b] + y, Ly, j, c.keepc, t == 0 || b != lane_block(*c.L, t - 1));
         R::apply(x, c.opx + R::FRAG + c.lane);
+        if (c.L->keep_half && ok) {
+            double* out = c.L->keep_half + (long)t * N * Ly + y;
+            each_value<N>(j, [&](int i, int n) { out[n * Ly] = x[i]; });
+        }
 #pragma unroll
         for (int i = 0; i < R::E; i++) x[i] = __dmul_rn(x[i], f[i]);
         R::apply(x, c.opx + R::FRAG + c.lane);
@@ -151,6 +155,18 @@ __device__ __forceinline__ void rows(const Chain& c, int t) {
                     const double h = f[i], v = __dmul_rn(x[i], h), u = __dmul_rn(w[n], __dmul_rn(h, h));
                     x[i] = div_rn(fma(4.0, v, -u), 3.0, 1.0 / 3.0);
                 });
+                if (c.L->keep_full && ok) {
+                    double* full = c.L->keep_full + (long)t * M + (long)r * N;
+                    each_value<N>(j, [&](int i, int n) { full[n] = w[n]; });
+                }
+                if (c.L->src_o) {
+                    const double wa = c.L->src_w[0][t + 1], wb = c.L->src_w[1][t + 1];
+                    const double *o = c.L->src_o + (long)(t + 1) * M + (long)r * N, *pa = c.L->src_p[0] + (long)r * N,
+                                 *pb = c.L->src_p[1] + (long)r * N;
+                    each_value<N>(j, [&](int i, int n) {
+                        x[i] = fma(fma(wa, __ldg(pa + n), wb * __ldg(pb + n)), __ldg(o + n), x[i]);
+                    });
+                }
             }
             double* out = c.L->hist + (long)(t + 1) * M + (long)r * N;
             if (ok) each_value<N>(j, [&](int i, int n) { out[n] = x[i]; });

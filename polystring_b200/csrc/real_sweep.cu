@@ -149,6 +149,10 @@ __device__ __forceinline__ void x_pass(const RealProblem& p, const double* fr, d
                     keep += 32 * R::E;
                 }
                 R::apply(x, fr + R::FRAG + lane);
+                if (L.keep_half && ok) {
+                    double* out = L.keep_half + (long)t * M + c;
+                    each_point<N>(j, [&](int k, int n) { out[n * P] = x[k]; });
+                }
 #pragma unroll
                 for (int i = 0; i < R::E; i++) x[i] = __dmul_rn(x[i], f[i]);
                 R::apply(x, fr + R::FRAG + lane);
@@ -235,6 +239,17 @@ __device__ __forceinline__ void plane_rows(const RealProblem& p, const double* f
                     const double v = __dmul_rn(q[i], h[i]), u = __dmul_rn(b[n], __dmul_rn(h[i], h[i]));
                     q[i] = div_rn(fma(4.0, v, -u), 3.0, 1.0 / 3.0);
                 });
+                if (L.keep_full && ok) {
+                    double* full = L.keep_full + (long)t * M + row;
+                    each_point<N>(j, [&](int i, int n) { full[n] = b[n]; });
+                }
+                if (L.src_o) {
+                    const double wa = L.src_w[0][t + 1], wb = L.src_w[1][t + 1];
+                    const double* o = L.src_o + (long)(t + 1) * M + row;
+                    each_point<N>(j, [&](int i, int n) {
+                        q[i] = fma(fma(wa, __ldg(L.src_p[0] + row + n), wb * __ldg(L.src_p[1] + row + n)), __ldg(o + n), q[i]);
+                    });
+                }
             }
             if (ok) each_point<N>(j, [&](int i, int n) { out[n] = q[i]; });
         }

@@ -18,6 +18,11 @@ struct RealLane {
     const double* eF[3];
     const double* eH[3];
     int sw[2];
+    // optional, one slice a step: the first half step before its factor,
+    // D' e^{-w ds/4} q, and the full step before its factor, D e^{-w ds/2} q
+    double *keep_half, *keep_full;
+    // optional source: slice t gets (src_w[0][t] src_p[0] + src_w[1][t] src_p[1]) src_o[t]
+    const double *src_p[2], *src_w[2], *src_o;
 };
 
 // One solve of a sweep: nl chains (one or two) of Ns contour steps.
