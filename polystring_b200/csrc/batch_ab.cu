@@ -1,8 +1,7 @@
 // batch_ab.cu -- many independent Model_AB solves, of uneven grid sizes,
 // contour lengths Ns, block fractions, cells and chiN, advanced together
 // (with, optionally, linear ABC triblock solves of model_abc.cu, which take
-// the same paths: shared generic sweeps on 32^3 / 48^3 / 64^3 grids, grouped
-// line passes on the others).
+// the same paths).
 //
 // The reference runs independent solves one per host thread
 // (scft/polystring_AB_backThread.cc); on one B200 a single small solve
@@ -13,18 +12,15 @@
 // Ns, so the active ones are a prefix), each CTA running the pass body of its
 // own solve (grouped_pass.cu).  Members are grouped by the number of grid
 // axes longer than one (2 or 3), which fixes the pass sequence of a step.
-// Solves on grids with a persistent sweep take it instead: 32^3 and 48^3
-// solves of one shape share one cooperative launch for all their contour
-// steps (sweep.cu, a descriptor per solve, the CTAs split between solves),
-// 64^3 solves run their own 64^3 sweep (sweep64.cu), which fills the GPU
-// alone (and so do 64^3 triblocks).  One batch iteration -- all propagators,
-// then every member's Q, densities and field update -- is captured once as a
-// CUDA graph and replayed.
+// Solves on grids with a persistent sweep take it instead: 2D solves in one
+// launch, a CTA a chain (plane_sweep.cu); 3D solves in launches that a cost
+// model picks, sharing the SMs or alone (real_sweep.cu).  One batch iteration --
+// all propagators, then every member's Q, densities and field update -- is
+// captured once as a CUDA graph and replayed.
 #include "batch_ab.h"
 
 #include <algorithm>
 #include <array>
-#include <map>
 #include <numeric>
 
 namespace ps {
@@ -122,77 +118,97 @@ void BatchAB::release() {
 
 BatchAB::~BatchAB() { release(); }
 
-void BatchAB::build_sweeps(const std::vector<int>& members) {
-    // shape -> solves, in member order
-    std::map<std::array<int, 3>, std::vector<int>> by_shape;
-    for (int k : members) {
-        if (k < (int)m_.size()) {
-            const ModelABParams& p = m_[k]->params();
-            by_shape[{p.Lx, p.Ly, p.Lz}].push_back(k);
-        } else {
-            const ModelABCParams& p = t_[k - m_.size()]->params();
-            by_shape[{p.Lx, p.Ly, p.Lz}].push_back(k);
+RealProblem BatchAB::sweep_descriptor(int k) const {
+    return k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
+}
+
+// one launch of the solves ks, per[i] CTAs a chain (3D)
+void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per) {
+    chunks_.emplace_back();
+    SweepChunk& c = chunks_.back();
+    c.n = (int)ks.size();
+    std::vector<RealProblem> d;
+    for (int k : ks) d.push_back(sweep_descriptor(k));
+    c.plane = d[0].Lz == 1;
+    if (c.plane) {
+        for (const RealProblem& p : d) c.pairs = std::max(c.pairs, plane_sweep_pairs(p.Lx, p.Ly));
+        for (const RealProblem& p : d) c.smem = std::max(c.smem, plane_sweep_smem(p, c.pairs));
+    } else {
+        PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * d.size()));
+        for (int i = 0; i < c.n; i++) {
+            d[i].bar = c.bar + 32 * (size_t)i;
+            d[i].cta0 = c.grid;
+            d[i].ncta = per[i];
+            c.grid += 2 * per[i];
+            c.smem = std::max(c.smem, real_sweep_smem(d[i]));
+            c.wide = c.wide || real_sweep_wide(d[i]);
         }
     }
-    for (auto& kv : by_shape) {
-        const int Lx = kv.first[0], Ly = kv.first[1], Lz = kv.first[2];
-        auto descriptor = [&](int k) {
-            return k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
-        };
-        int nfrag = 0;
-        for (int k : kv.second) nfrag = std::max(nfrag, descriptor(k).nfrag);
-        auto emplace = [&](int i0, int n, int per, const std::vector<int>& ks) {
-            chunks_.emplace_back();
-            SweepChunk& c = chunks_.back();
-            c.Lx = Lx; c.Ly = Ly; c.Lz = Lz; c.nfrag = nfrag;
-            c.n = n;
-            c.per = per;
-            PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * (size_t)n));
-            std::vector<RealProblem> d(n);
-            for (int i = 0; i < n; i++) {
-                d[i] = descriptor(ks[i0 + i]);
-                d[i].bar = c.bar + 32 * (size_t)i;
-                d[i].cta0 = 2 * i * per;
-                d[i].ncta = per;
-            }
-            PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
-            PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
-        };
-        if (Lz == 1) {
-            // 2D solves: a CTA a chain, independent of each other, longest first
-            std::vector<int> ks = kv.second;
-            std::stable_sort(ks.begin(), ks.end(), [&](int a, int b) { return Ns_of(a) > Ns_of(b); });
-            emplace(0, (int)ks.size(), 0, ks);
+    PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
+    PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+}
+
+void BatchAB::build_sweeps(const std::vector<int>& members) {
+    // 2D solves: a CTA a chain, independent of each other, one launch
+    std::vector<int> planes, ks;
+    for (int k : members) (sweep_descriptor(k).Lz == 1 ? planes : ks).push_back(k);
+    auto longer = [&](int a, int b) { return Ns_of(a) > Ns_of(b); };
+    std::stable_sort(planes.begin(), planes.end(), longer);
+    if (!planes.empty()) add_chunk(planes, {});
+    // 3D solves: a launch lasts its longest solve's Ns steps.  A step of a solve
+    // alone takes about 5 us for its two barriers and phases' latencies and
+    // 24 ps a point and chain (7.4, 12.4, 17.6 us at 32^3, 48^3, 64^3); one of a
+    // shared launch 5 us and 32 ps a point and chain of all its solves (22.9 us
+    // for nine of 32^3, 24.2 for three of 48^3, 34.4 for two of 64^3).  With the
+    // solves in order of Ns, then size, the launches are consecutive runs of
+    // that order; pick the runs with the least total time (dynamic programme).
+    std::stable_sort(ks.begin(), ks.end(), [&](int a, int b) {
+        return Ns_of(a) != Ns_of(b) ? Ns_of(a) > Ns_of(b) : points_of(a) > points_of(b);
+    });
+    const int nk = (int)ks.size();
+    const int most = real_sweep_resident(0, true) / 2;   // solves of a launch: a CTA a chain at least
+    std::vector<double> best(nk + 1, 0.0);
+    std::vector<int> from(nk + 1, 0);
+    for (int i = 1; i <= nk; i++) {
+        best[i] = -1.0;
+        double points = 0.0;
+        for (int j = i - 1; j >= std::max(0, i - most); j--) {
+            points += 2.0 * points_of(ks[j]);
+            const double c = best[j] + Ns_of(ks[j]) * (5.0 + (i - j == 1 ? 2.4e-5 : 3.2e-5) * points);
+            if (best[i] < 0.0 || c < best[i]) { best[i] = c; from[i] = j; }
+        }
+    }
+    std::vector<std::pair<int, int>> runs;   // [i0, i1) in ks
+    for (int i = nk; i > 0; i = from[i]) runs.push_back({from[i], i});
+    std::reverse(runs.begin(), runs.end());
+    for (const auto& run : runs) {
+        const std::vector<int> part(ks.begin() + run.first, ks.begin() + run.second);
+        if (part.size() == 1) {
+            own_.push_back(part[0]);   // as alone: a CTA an SM, factors in shared memory
             continue;
         }
-        const int resident = real_sweep_prepare(Lx, Ly, Lz, nfrag, true);
-        const int tasks = real_sweep_tasks(Lx, Ly, Lz);
-        // A launch of n solves gives each per = resident / n CTAs (at most the
-        // tasks of a phase) and lasts its longest solve's Ns steps, each step
-        // sweep_rounds_per_step(per) rounds of tasks.  With the solves in
-        // order of Ns, the launches are consecutive runs of that order; pick
-        // the runs with the least total cost (dynamic programme over n).
-        std::vector<int> ks = kv.second;
-        std::stable_sort(ks.begin(), ks.end(), [&](int a, int b) { return Ns_of(a) > Ns_of(b); });
-        const int nk = (int)ks.size();
-        auto per_of = [&](int n) { return std::max(1, std::min(tasks, resident / 2 / n)); };
-        std::vector<double> best(nk + 1, 0.0);
-        std::vector<int> from(nk + 1, 0);
-        for (int i = 1; i <= nk; i++) {
-            best[i] = -1.0;
-            for (int j = std::max(0, i - resident / 2); j < i; j++) {
-                const double c = best[j] + (double)Ns_of(ks[j]) * real_sweep_step_cost(Lx, Ly, Lz, per_of(i - j));
-                if (best[i] < 0.0 || c < best[i]) { best[i] = c; from[i] = j; }
-            }
+        // CTAs in proportion to the solves' points, no more than their tasks
+        size_t smem = 0;
+        bool wide = false;
+        double points = 0.0;
+        for (int k : part) {
+            const RealProblem p = sweep_descriptor(k);
+            smem = std::max(smem, real_sweep_smem(p));
+            wide = wide || real_sweep_wide(p);
+            points += points_of(k);
         }
-        std::vector<std::pair<int, int>> runs;   // [i0, i1) in ks
-        for (int i = nk; i > 0; i = from[i]) runs.push_back({from[i], i});
-        std::reverse(runs.begin(), runs.end());
-        for (const auto& run : runs) {
-            const int n = run.second - run.first;
-            emplace(run.first, n, per_of(n), ks);
+        const int half = real_sweep_resident(smem, wide) / 2, spare = half - (int)part.size();
+        std::vector<int> per;
+        for (int k : part) {
+            const RealProblem p = sweep_descriptor(k);
+            per.push_back(std::min(real_sweep_tasks(p.Lx, p.Ly, p.Lz), 1 + (int)(spare * (points_of(k) / points))));
         }
+        add_chunk(part, per);
     }
+}
+
+double BatchAB::points_of(int k) const {
+    return (double)(k < (int)m_.size() ? m_[k]->M() : t_[k - m_.size()]->M());
 }
 
 PairChain* BatchAB::chain_of(int k) const {
@@ -270,12 +286,17 @@ void BatchAB::build_group(Group& g) {
 void BatchAB::enqueue_iteration() {
     int launches = 0;
     for (const SweepChunk& c : chunks_) {
-        if (c.Lz == 1) {
-            plane_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.nfrag, st_);
+        if (c.plane) {
+            plane_sweep_launch_many(c.dev, c.n, c.pairs, c.smem, st_);
         } else {
             PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-            real_sweep_launch_many(c.dev, c.n, c.Lx, c.Ly, c.Lz, c.nfrag, 2 * c.per * c.n, st_);
+            real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
         }
+        launches++;
+    }
+    for (int k : own_) {
+        if (k < (int)m_.size()) m_[k]->enqueue_propagate(st_);
+        else t_[k - (int)m_.size()]->enqueue_propagate(st_);
         launches++;
     }
     int Ns_max = 0;

@@ -40,10 +40,12 @@ private:
         std::vector<int> prefix[9];
         size_t smem[9] = {};
     };
-    // solves of one shape with a generic persistent sweep, in one cooperative
-    // launch: n descriptors on the device, per CTAs a solve, n x 32 barrier words
+    // solves that share a sweep launch: their descriptors on the device, and
+    // 32 barrier words each (3D)
     struct SweepChunk {
-        int Lx = 0, Ly = 0, Lz = 0, nfrag = 0, per = 0, n = 0;
+        int n = 0, grid = 0, pairs = 0;
+        bool plane = false, wide = false;
+        size_t smem = 0;
         RealProblem* dev = nullptr;
         unsigned* bar = nullptr;
     };
@@ -51,6 +53,9 @@ private:
     GroupSolve describe(int k) const;   // grouped-pass descriptor of member k
     PairChain* chain_of(int k) const;
     int Ns_of(int k) const;
+    double points_of(int k) const;
+    RealProblem sweep_descriptor(int k) const;
+    void add_chunk(const std::vector<int>& ks, const std::vector<int>& per);
     void build_sweeps(const std::vector<int>& members);
     void release();
     void enqueue_iteration();
@@ -58,6 +63,7 @@ private:
     std::vector<ModelABC*> t_;
     std::vector<Group> groups_;
     std::vector<SweepChunk> chunks_;
+    std::vector<int> own_;                   // solves propagated by their own sweep launch
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t graph_ = nullptr;
     int launches_ = 0, launches_prop_ = 0;

@@ -393,16 +393,11 @@ bool plane_line_ok(int N) {
     return false;
 }
 
-size_t plane_smem(int Lx, int Ly, int nfrag) {
-    const size_t nt = std::max(tiles_of(Lx), tiles_of(Ly));
-    return sizeof(double) * ((size_t)nfrag + 2 * (size_t)Lx * pitch_of(Ly) + nt * 32 * (values_of(Lx) + values_of(Ly)));
-}
+int pairs_of(int Lx, int Ly) { return std::max(tiles_of(Lx), tiles_of(Ly)); }
 
-void plane_launch(const RealProblem& one, const RealProblem* many, int nchains, int Lx, int Ly, int nfrag,
-                  cudaStream_t st) {
-    const int threads = 64 * std::max(tiles_of(Lx), tiles_of(Ly));
-    plane_sweep_kernel<<<nchains, threads, plane_smem(Lx, Ly, nfrag), st>>>(one, many);
-    PS_CUDA(cudaGetLastError());
+size_t plane_smem(int Lx, int Ly, int nfrag, int pairs) {
+    return sizeof(double) *
+           ((size_t)nfrag + 2 * (size_t)Lx * pitch_of(Ly) + (size_t)pairs * 32 * (values_of(Lx) + values_of(Ly)));
 }
 
 #define LN_CASES(X) PL_CASES(X) X(96) X(128) X(192) X(256) X(352)
@@ -411,21 +406,27 @@ void plane_launch(const RealProblem& one, const RealProblem* many, int nchains, 
 
 bool plane_sweep_supported(int Lx, int Ly) {
     return plane_line_ok(Lx) && plane_line_ok(Ly) &&
-           plane_smem(Lx, Ly, 2 * (real_frag_doubles(Lx) + real_frag_doubles(Ly))) <= kSmemLimit;
+           plane_smem(Lx, Ly, 2 * (real_frag_doubles(Lx) + real_frag_doubles(Ly)), kMaxLine / 8) <= kSmemLimit;
 }
 
 void plane_sweep_prepare() {
     PS_CUDA(cudaFuncSetAttribute(plane_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
 }
 
+int plane_sweep_pairs(int Lx, int Ly) { return pairs_of(Lx, Ly); }
+size_t plane_sweep_smem(const RealProblem& p, int pairs) { return plane_smem(p.Lx, p.Ly, p.nfrag, pairs); }
+
 void plane_sweep_launch(const RealProblem& p, cudaStream_t st) {
-    plane_launch(p, nullptr, p.nl, p.Lx, p.Ly, p.nfrag, st);
+    const int pairs = pairs_of(p.Lx, p.Ly);
+    plane_sweep_kernel<<<p.nl, 64 * pairs, plane_sweep_smem(p, pairs), st>>>(p, nullptr);
+    PS_CUDA(cudaGetLastError());
 }
 
-void plane_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int nfrag, cudaStream_t st) {
+void plane_sweep_launch_many(const RealProblem* d, int n, int pairs, size_t smem, cudaStream_t st) {
     RealProblem one{};
     one.nl = 2;
-    plane_launch(one, d, 2 * n, Lx, Ly, nfrag, st);
+    plane_sweep_kernel<<<2 * n, 64 * pairs, smem, st>>>(one, d);
+    PS_CUDA(cudaGetLastError());
 }
 
 bool line_sweep_supported(int Lx) {

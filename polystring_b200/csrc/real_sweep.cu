@@ -486,32 +486,31 @@ bool real_sweep_supported(int Lx, int Ly, int Lz) {
            smem_bytes(Ly, Lz, 2 * (real_frag_doubles(Lx) + real_frag_doubles(Ly) + real_frag_doubles(Lz))) <= kSmemLimit;
 }
 
-int real_sweep_prepare(int Lx, int Ly, int Lz, int nfrag, bool shared) {
-    const size_t smem = smem_bytes(Ly, Lz, nfrag);
-    int dev = 0, sms = 0, occ = 0;
+size_t real_sweep_smem(const RealProblem& p) { return smem_bytes(p.Ly, p.Lz, p.nfrag); }
+bool real_sweep_wide(const RealProblem& p) { return wide(p.Lx, p.Ly, p.Lz); }
+
+// sets the kernels' attributes; the SMs of the device
+static int prepare_kernels() {
+    int dev = 0, sms = 0;
     PS_CUDA(cudaGetDevice(&dev));
     PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     PS_CUDA(cudaFuncSetAttribute(real_sweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
     PS_CUDA(cudaFuncSetAttribute(real_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
-    if (shared && !wide(Lx, Ly, Lz))
-        PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, real_sweep_kernel<false>, kNT, smem));
-    else
-        PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, real_sweep_kernel<true>, kNT, smem));
+    return sms;
+}
+
+int real_sweep_resident(size_t smem, bool one) {
+    const int sms = prepare_kernels();
+    int occ = 0;
+    if (one) PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, real_sweep_kernel<true>, kNT, smem));
+    else PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, real_sweep_kernel<false>, kNT, smem));
     if (occ < 1) throw Error(-2, "sweep kernel does not fit on an SM");
-    return sms * (shared ? occ : 1);
+    return sms * occ;
 }
 
 int real_sweep_tasks(int Lx, int Ly, int Lz) {
     const int xt = 2 * ((Ly * Lz + 7) / 8);
     return std::max(Lx, (xt + kNT / 32 - 1) / (kNT / 32));
-}
-
-double real_sweep_step_cost(int Lx, int Ly, int Lz, int per) {
-    if (per < 1) per = 1;
-    const int warps = kNT / 32;
-    const int xt = 2 * ((Ly * Lz + 7) / 8);
-    const double rounds_x = (xt + per * warps - 1) / (per * warps), rounds_p = (Lx + per - 1) / per;
-    return 1.0 + rounds_x + rounds_p;
 }
 
 int real_sweep_columns(int variant) { return 8 << variant; }
@@ -532,9 +531,8 @@ void real_sweep_launch(const RealProblem& p0, int ncta, cudaStream_t st) {
     launch(p, nullptr, 0, smem, true, ncta * p.nl, st);
 }
 
-void real_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int Lz, int nfrag, int grid,
-                            cudaStream_t st) {
-    launch(RealProblem{}, d, n, smem_bytes(Ly, Lz, nfrag), wide(Lx, Ly, Lz), grid, st);
+void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool one, int grid, cudaStream_t st) {
+    launch(RealProblem{}, d, n, smem, one, grid, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -555,8 +553,7 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     const std::vector<double> f = real_operator_tables(n, k, ds, dim_ == 1, fo_);
     nfrag_ = (int)f.size();
     if (dim_ == 3) {
-        ncta_ = std::max(1, std::min(real_sweep_prepare(n[0], n[1], n[2], nfrag_, false) / nl,
-                                     real_sweep_tasks(n[0], n[1], n[2])));
+        ncta_ = std::max(1, std::min(prepare_kernels() / nl, real_sweep_tasks(n[0], n[1], n[2])));
         PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
     } else if (dim_ == 2) {
         plane_sweep_prepare();

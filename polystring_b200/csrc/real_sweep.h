@@ -47,29 +47,31 @@ std::vector<double> real_operator_tables(const int n[3], const double k[3], doub
 
 // whether a 3D grid has this sweep
 bool real_sweep_supported(int Lx, int Ly, int Lz);
-// sets kernel attributes; returns the CTAs of one solve alone (one an SM), or
-// with `shared` those that a shared launch can have resident at once, with nfrag
-// doubles of fragments
-int real_sweep_prepare(int Lx, int Ly, int Lz, int nfrag, bool shared);
 // CTAs one chain can keep busy
 int real_sweep_tasks(int Lx, int Ly, int Lz);
-// time of a contour step with `per` CTAs a chain, in units of a shared-launch cost model
-double real_sweep_step_cost(int Lx, int Ly, int Lz, int per);
+// shared memory of a solve in a shared launch; whether it needs the kernel of
+// one CTA an SM; CTAs resident at once in a shared launch of such solves
+size_t real_sweep_smem(const RealProblem& p);
+bool real_sweep_wide(const RealProblem& p);
+int real_sweep_resident(size_t smem, bool wide);
 // x-tile variants (columns a task; same arithmetic)
 constexpr int kRealVariants = 3;
 int real_sweep_columns(int variant);
 // ncta CTAs a chain
 void real_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
-// n solves of one shape described in device memory, grid CTAs in all, nfrag the
-// largest of the solves'
-void real_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int Lz, int nfrag, int grid, cudaStream_t st);
+// n solves described in device memory (shapes may differ), grid CTAs in all, the
+// largest of the solves' shared memory
+void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool wide, int grid, cudaStream_t st);
 
 // 2D grids of up to 64 x 64 points, one CTA a chain
 bool plane_sweep_supported(int Lx, int Ly);
 void plane_sweep_prepare();
 void plane_sweep_launch(const RealProblem& p, cudaStream_t st);
-// n solves of two chains and one shape described in device memory
-void plane_sweep_launch_many(const RealProblem* d, int n, int Lx, int Ly, int nfrag, cudaStream_t st);
+// n solves of two chains described in device memory (shapes may differ): the
+// largest of their warp pairs and of their shared memory
+int plane_sweep_pairs(int Lx, int Ly);
+size_t plane_sweep_smem(const RealProblem& p, int pairs);
+void plane_sweep_launch_many(const RealProblem* d, int n, int pairs, size_t smem, cudaStream_t st);
 // 1D grids
 bool line_sweep_supported(int Lx);
 void line_sweep_launch(const RealProblem& p, cudaStream_t st);
@@ -91,7 +93,6 @@ public:
     // PS_B200_SWEEP_VARIANT=v forces variant v)
     void tune(const RealProblem& p, cudaStream_t st);
     void enqueue(const RealProblem& p, cudaStream_t st) const;
-    int fragments() const { return nfrag_; }   // doubles of the operators
     int error(cudaStream_t st) const;   // barrier error flag (synchronises)
 
 private:

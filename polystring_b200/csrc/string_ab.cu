@@ -301,7 +301,9 @@ void StringAB::enqueue_scft_iteration() {
     double *wa = wa_.p + off, *wb = wb_.p + off, *phiA = phiA_.p + off, *phiB = phiB_.p + off;
     double* scal = scal_.p + 8 * lo_;
     if (real_) {
-        plane_sweep_launch_many(images_, nloc_, p_.Lx, p_.Ly, real_->fragments(), st_);
+        const int pairs = plane_sweep_pairs(p_.Lx, p_.Ly);
+        const RealLane none[2] = {};
+        plane_sweep_launch_many(images_, nloc_, pairs, plane_sweep_smem(real_->problem(none, Ns_), pairs), st_);
     } else if (use_cluster_) {
         SweepArgs a{};
         a.hf = hf_.p; a.hc = hc_.p;
