@@ -14,6 +14,8 @@
 //               ramp 1 - lambda^(k+1), ring position update     (one block, shared memory)
 //   ax_combine  W = w(cur) + sum C (w(kk) - w(cur)), D likewise,
 //               w(cur') = W + ramp D, plus the next Boltzmann factors
+#include <algorithm>
+
 #include "ps_internal.h"
 #include "field_kernels.h"
 #include "anderson.h"
@@ -76,6 +78,7 @@ __global__ void __launch_bounds__(kRedThreads) ax_dots_kernel(AXArgs a, double* 
     const int nn = s->k < n ? s->k : n;
     const long M = a.M;
     const int j0 = blockIdx.y * kJC;
+    if (j0 > nn) return;   // no such sums yet: the solve reads j <= nn only
     const double* dF[3] = {a.dA, a.dB, NF == 3 ? a.dC : a.dA};
     double acc[NF * kJC];
 #pragma unroll
@@ -129,11 +132,16 @@ __global__ void __launch_bounds__(kRedThreads) ax_solve_kernel(AXArgs a, const d
     __shared__ double sB[NF][(NMAX + 1) * (NMAX + 1)];
     __shared__ double U[NMAX * NMAX], V[NMAX], C[NMAX], F[NMAX];
     __shared__ int piv_row, singular;
-    // fixed-order reduction of the partial sums
-    for (int j = tid; j < NF * NMAX; j += nt) {
+    // fixed-order reduction of the partial sums, a warp a sum (one thread a sum
+    // waited for G loads in a row: the Anderson step of a small grid took 40 us)
+    for (int j = tid >> 5; j < NF * NMAX; j += nt >> 5) {
+        if (j % NMAX > nn) continue;
         double t = 0.0;
-        for (int b = 0; b < G; b++) t += partial[(long)b * NF * NMAX + j];
-        row[j] = t / (double)a.M;
+#pragma unroll 5
+        for (int b = tid & 31; b < G; b += 32) t += partial[(long)b * NF * NMAX + j];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if ((tid & 31) == 0) row[j] = t / (double)a.M;
     }
     double* BG[3] = {a.BA, a.BB, a.BC};
     for (int f = 0; f < NF; f++)
@@ -183,15 +191,21 @@ __global__ void __launch_bounds__(kRedThreads) ax_solve_kernel(AXArgs a, const d
     }
     __syncthreads();
     for (int k = 0; k < nn; k++) {
-        if (tid == 0) {
-            int p = k;
-            double best = fabs(U[k * nn + k]);
-            for (int i = k + 1; i < nn; i++) {
-                const double v = fabs(U[i * nn + k]);
-                if (v > best) { best = v; p = i; }
+        if (tid < 32) {   // the first row of the largest |U[i][k]| (nn < 32: a lane a row)
+            double best = tid >= k && tid < nn ? fabs(U[tid * nn + k]) : -1.0;
+            if (best != best) best = -1.0;   // a NaN exceeds nothing
+            int p = tid;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double v = __shfl_xor_sync(0xffffffffu, best, o);
+                const int r = __shfl_xor_sync(0xffffffffu, p, o);
+                if (v > best || (v == best && r < p)) { best = v; p = r; }
             }
-            piv_row = p;
-            if (best == 0.0) singular = 1;
+            if (tid == 0) {
+                const bool nan = U[k * nn + k] != U[k * nn + k];   // and nothing exceeds one in row k
+                piv_row = nan ? k : p;
+                if (!nan && best == 0.0) singular = 1;
+            }
         }
         __syncthreads();
         if (singular) break;
@@ -319,8 +333,10 @@ int ax_nmax(int n) {
 
 template <int NF, int NMAX>
 void launch_ax_nf(const AXArgs& a, double* partial, cudaStream_t st) {
-    ax_dots_kernel<NF, NMAX><<<dim3(kRedBlocks, (NMAX + kJC) / kJC), kRedThreads, 0, st>>>(a, partial);
-    ax_solve_kernel<NF, NMAX><<<1, kRedThreads, 0, st>>>(a, partial, kRedBlocks);
+    // small grids fill fewer blocks
+    const int G = (int)std::min((long)kRedBlocks, (a.M + kRedThreads - 1) / kRedThreads);
+    ax_dots_kernel<NF, NMAX><<<dim3(G, (NMAX + kJC) / kJC), kRedThreads, 0, st>>>(a, partial);
+    ax_solve_kernel<NF, NMAX><<<1, kRedThreads, 0, st>>>(a, partial, G);
 }
 
 template <int NF>

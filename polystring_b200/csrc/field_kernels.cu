@@ -171,23 +171,39 @@ struct ArcF {
 // density
 // ---------------------------------------------------------------------------
 // phi[m] = (cc * ds) * sum_{s=0}^{n} c_s q[s][m] qc[n-s][m]; cc = 1/Q from
-// device memory when Qdev != nullptr, else cc_host.
-__global__ void density_kernel(const double* __restrict__ q, const double* __restrict__ qc, int n, long M,
-                               const double* __restrict__ c, double ds, const double* Qdev, double cc_host,
-                               double* __restrict__ phi, long bstride_q, long bstride_phi, const double* Qbatch) {
+// device memory when Qdev != nullptr, else cc_host.  HBM bound (16 B a point and
+// slice): a block takes 32 points, its eight warps every eighth slice each, so
+// that small grids (64 points of 1D to 64^2) also have some slices in flight at
+// once instead of one thread's serial chain; the warps' sums are added in order.
+constexpr int kDensityWarps = 8;
+__global__ void __launch_bounds__(32 * kDensityWarps) density_kernel(
+    const double* __restrict__ q, const double* __restrict__ qc, int n, long M, const double* __restrict__ c, double ds,
+    const double* Qdev, double cc_host, double* __restrict__ phi, long bstride_q, long bstride_phi,
+    const double* Qbatch) {
     const long b = blockIdx.y;
     q += b * bstride_q;
     qc += b * bstride_q;
     phi += b * bstride_phi;
-    double cc = cc_host;
-    if (Qdev) cc = 1.0 / Qdev[0];
-    if (Qbatch) cc = 1.0 / Qbatch[b * 8];
-    const double scale = cc * ds;
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < M; m += stride) {
-        double acc = 0.0;
-        for (int s = 0; s <= n; s++) acc += c[s] * (q[(long)s * M + m] * qc[(long)(n - s) * M + m]);
-        phi[m] = acc * scale;
+    __shared__ double part[kDensityWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long m = (long)blockIdx.x * 32 + lane;
+    double acc = 0.0;
+    if (m < M) {
+        const double* f = q + m;
+        const double* r = qc + (long)n * M + m;
+#pragma unroll 4
+        for (int s = warp; s <= n; s += kDensityWarps) acc += c[s] * (f[(long)s * M] * r[-(long)s * M]);
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && m < M) {
+        double cc = cc_host;
+        if (Qdev) cc = 1.0 / Qdev[0];
+        if (Qbatch) cc = 1.0 / Qbatch[b * 8];
+        double t = part[0][lane];
+#pragma unroll
+        for (int w = 1; w < kDensityWarps; w++) t += part[w][lane];
+        phi[m] = t * (cc * ds);
     }
 }
 
@@ -330,8 +346,8 @@ void launch_arc_sq(const double* a, const double* b, long M, double* partial, do
 void launch_density(const double* q, const double* qc, int n, long M, const double* c, double ds,
                     const double* Qdev, double cc_host, double* phi, int nbatch, long bstride_q, long bstride_phi,
                     const double* Qbatch, cudaStream_t st) {
-    dim3 grid(grid_for(M), nbatch);
-    density_kernel<<<grid, 256, 0, st>>>(q, qc, n, M, c, ds, Qdev, cc_host, phi, bstride_q, bstride_phi, Qbatch);
+    dim3 grid((unsigned)((M + 31) / 32), nbatch);
+    density_kernel<<<grid, 32 * kDensityWarps, 0, st>>>(q, qc, n, M, c, ds, Qdev, cc_host, phi, bstride_q, bstride_phi, Qbatch);
     PS_CUDA(cudaGetLastError());
 }
 
