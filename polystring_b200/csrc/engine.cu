@@ -475,7 +475,7 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
         real_->tune(sweep_descriptor(), st_);
     }
     PS_CUDA(cudaStreamSynchronize(st_));
-    launches_per_prop_ = real_ ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
+    launches_per_prop_ = real_ || chain_->small_etd() ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
     launches_per_iter_ = launches_per_prop_ + 2 + 2 + (p.scft == 1 ? 4 : 1);
 }
 

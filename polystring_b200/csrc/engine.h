@@ -124,6 +124,8 @@ public:
     void autotune(cudaStream_t st);
     // kernel launches per pair step
     int launches_per_step() const;
+    // ETDRK4: whether all steps run in one launch
+    bool small_etd() const;
     long M() const { return M_; }
     const AxisPlan& plan() const { return plan_; }
     // work fields and tables (for grouped launches over many chains)

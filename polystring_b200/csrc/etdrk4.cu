@@ -13,14 +13,17 @@
 // with E = exp(ds L), E2 = exp(ds L / 2) and L = -k^2 (calc_k2_orthogonal).
 // Every spectral operation multiplies by real tables that are even in k, so
 // the packed field carries both lanes' spectra at once; the nonlinear term
-// takes each lane's own w.  The transforms are the line passes of
-// line_pass.cu (MODE_FWD / MODE_INV over every axis); the elementwise work
-// of the step is in the kernels below.
+// takes each lane's own w.  Grids of up to 4096 points of 1D and 2D run all
+// steps in one CTA (etd_small_kernel); on others the transforms are the line
+// passes of line_pass.cu (MODE_FWD / MODE_INV over every axis) and the
+// elementwise work of the step is in the kernels below.
 #include "engine.h"
+#include "fft_core.cuh"
 #include "ps_internal.h"
 
 #include <cmath>
 #include <complex>
+#include <cstdlib>
 
 namespace ps {
 
@@ -107,6 +110,218 @@ __global__ void etd_store_kernel(const double2* __restrict__ T, double* __restri
     }
 }
 
+// ---------------------------------------------------------------------------
+// small grids: all steps in one CTA
+// ---------------------------------------------------------------------------
+// The packed field ping-pongs between two shared-memory buffers, one Stockham
+// radix pass a barrier; element (x, y) sits at x P + y with an odd pitch P, so
+// that threads on consecutive lines of either axis fall in different banks.
+// The spectral fields of a point belong to one thread for the whole solve: in
+// registers up to 4 points a thread, else in the chain's scratch fields.
+// What bounds it is the chain of 8 transforms a step, each radix pass some 400
+// cycles of shared-memory and FP64 latency and a barrier: 32^2 16.7 us a step,
+// 1D 64 points 5.0 us (by line passes 33 and 17 launches, 59 and 33 us).
+constexpr long kSmallPoints = 4096;
+
+struct EtdSmall {
+    double *hf, *hc;              // histories; hc == nullptr: lane c carries nothing
+    const double *wf[2], *wc[2];  // w of each lane before and from its switch step
+    int swf, swc, nsteps, Lx, Ly;
+    const double *E, *E2, *Q, *f1, *f2, *f3;
+    double2 *V, *Nv, *A, *S;      // scratch fields (more than 4 points a thread)
+    const double2 *twx, *twy;
+};
+
+extern __shared__ __align__(16) double2 esm[];
+
+// nl lines of one axis: line l, element n at l ls + n es; magic: ceil(2^32 / nl),
+// so that b / nl is the high word of b magic for b < 2^16
+struct SmallAxis {
+    int N, nl, ls, es, tw;
+    unsigned magic;
+};
+
+// one radix pass of every line, from offset `in` of the shared memory to `out`
+template <int N, int R, int NS, int SIGN, int NT>
+__device__ __forceinline__ void small_pass(int in, int out, const SmallAxis& g) {
+    constexpr int NB = N / R;
+    for (int b = threadIdx.x; b < g.nl * NB; b += NT) {
+        const int j = g.nl == 1 ? b : (int)__umulhi((unsigned)b, g.magic), l = b - j * g.nl, jm = j % NS;
+        const double2* src = esm + in + l * g.ls + j * g.es;
+        double2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = src[r * NB * g.es];
+        if (NS > 1) {
+#pragma unroll
+            for (int r = 1; r < R; r++) {
+                double2 w = esm[g.tw + (jm * r * (N / (NS * R))) % N];
+                if (SIGN > 0) w.y = -w.y;
+                v[r] = cmul(v[r], w);
+            }
+        }
+        Dft<R, SIGN>::run(v);
+        double2* dst = esm + out + l * g.ls + ((j / NS) * NS * R + jm) * g.es;
+#pragma unroll
+        for (int r = 0; r < R; r++) dst[r * NS * g.es] = v[r];
+    }
+    __syncthreads();
+}
+// transform of every line of the field at offset a (the other buffer at b);
+// returns whether the field has changed places
+template <int N, int SIGN, int NT>
+__device__ __forceinline__ bool small_lines(int a, int b, const SmallAxis& g) {
+    using P = Plan<N>;
+    if constexpr (P::P >= 1) small_pass<N, P::r0, 1, SIGN, NT>(a, b, g);
+    if constexpr (P::P >= 2) small_pass<N, P::r1, P::r0, SIGN, NT>(b, a, g);
+    if constexpr (P::P >= 3) small_pass<N, P::r2, P::r0 * P::r1, SIGN, NT>(a, b, g);
+    return P::P % 2 == 1;
+}
+template <int SIGN, int NT>
+__device__ __forceinline__ bool small_axis(int a, int b, const SmallAxis& g) {
+    switch (g.N) {
+#define X(V) case V: return small_lines<V, SIGN, NT>(a, b, g);
+        X(2) X(4) X(8) X(12) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(352)
+#undef X
+    }
+    return false;
+}
+
+template <int NT, int KP>
+__global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant__ EtdSmall a) {
+    // the spectral fields in registers, and with the registers of up to 256
+    // threads the tables and w as well (read from the L2 twice a stage otherwise)
+    constexpr bool REGS = KP <= 4, TAB = REGS && NT <= 256;
+    const int M = a.Lx * a.Ly, P = a.Ly | 1, F = a.Lx * P;
+    auto magic = [](int n) { return (unsigned)(((1ull << 32) + n - 1) / n); };
+    const SmallAxis ax = {a.Lx, a.Ly, 1, P, 0, magic(a.Ly)}, ay = {a.Ly, a.Lx, P, 1, a.Lx, magic(a.Lx)};
+    int cur = a.Lx + a.Ly, oth = cur + F;   // the field, the other buffer
+    for (int i = threadIdx.x; i < a.Lx; i += NT) esm[i] = a.twx[i];
+    if (a.Ly > 1)
+        for (int i = threadIdx.x; i < a.Ly; i += NT) esm[a.Lx + i] = a.twy[i];
+    const double Md = (double)M, rM = 1.0 / Md;
+    const bool pow2 = (M & (M - 1)) == 0;
+    double2 rV[REGS ? KP : 1], rN[REGS ? KP : 1], rA[REGS ? KP : 1], rS[REGS ? KP : 1];
+    int place[KP];
+#pragma unroll
+    for (int k = 0; k < KP; k++) {
+        const int m = threadIdx.x + k * NT, x = m / a.Ly;
+        place[k] = x * P + (m - x * a.Ly);
+    }
+    auto each = [&](auto f) {   // this thread's points: (slot, point, place in the buffers)
+#pragma unroll
+        for (int k = 0; k < KP; k++) {
+            const int m = threadIdx.x + k * NT;
+            if (m < M) f(k, m, place[k]);
+        }
+    };
+    auto V = [&](int k, int m) -> double2& { if constexpr (REGS) return rV[k]; else return a.V[m]; };
+    auto Nv = [&](int k, int m) -> double2& { if constexpr (REGS) return rN[k]; else return a.Nv[m]; };
+    auto A = [&](int k, int m) -> double2& { if constexpr (REGS) return rA[k]; else return a.A[m]; };
+    auto S = [&](int k, int m) -> double2& { if constexpr (REGS) return rS[k]; else return a.S[m]; };
+    auto flip = [&](bool moved) {
+        if (moved) {
+            const int c = cur;
+            cur = oth;
+            oth = c;
+        }
+    };
+    auto forward = [&]() {
+        __syncthreads();
+        if (a.Ly > 1) flip(small_axis<-1, NT>(cur, oth, ay));
+        flip(small_axis<-1, NT>(cur, oth, ax));
+    };
+    auto inverse = [&]() {
+        __syncthreads();
+        flip(small_axis<+1, NT>(cur, oth, ax));
+        if (a.Ly > 1) flip(small_axis<+1, NT>(cur, oth, ay));
+    };
+    double2 q[REGS ? KP : 1];   // the slice (more points: read back from the history)
+    double tab[6][TAB ? KP : 1], w[2][TAB ? KP : 1];
+    const double* const tabs[6] = {a.E, a.E2, a.Q, a.f1, a.f2, a.f3};
+    if constexpr (TAB)
+#pragma unroll
+        for (int i = 0; i < 6; i++) each([&](int k, int m, int) { tab[i][k] = __ldg(tabs[i] + m); });
+    auto T = [&](int i, int k, int m) { if constexpr (TAB) return tab[i][k]; else return __ldg(tabs[i] + m); };
+    for (int t = 0; t < a.nsteps; t++) {
+        const double *qf = a.hf + (long)t * M, *qc = a.hc ? a.hc + (long)t * M : nullptr;
+        const double *wf = a.wf[t >= a.swf], *wc = a.wc[t >= a.swc];
+        if constexpr (TAB)
+            if (t == 0 || t == a.swf || t == a.swc)
+                each([&](int k, int m, int) {
+                    w[0][k] = __ldg(wf + m);
+                    w[1][k] = __ldg(wc + m);
+                });
+        auto W = [&](int i, int k, int m) { if constexpr (TAB) return w[i][k]; else return __ldg((i ? wc : wf) + m); };
+        if (t == 0 || t == a.swf || t == a.swc) {
+            each([&](int, int m, int i) { esm[cur + i] = make_double2(qf[m], qc ? qc[m] : 0.0); });
+            forward();
+            each([&](int k, int m, int i) { V(k, m) = esm[cur + i]; });
+        }
+        each([&](int k, int m, int i) {
+            double2 x;
+            if (!REGS || t == 0) x = make_double2(qf[m], qc ? qc[m] : 0.0);
+            else x = q[REGS ? k : 0];
+            esm[cur + i] = make_double2(-W(0, k, m) * x.x, qc ? -W(1, k, m) * x.y : 0.0);
+        });
+#pragma unroll 1
+        for (int stage = 0; stage < 4; stage++) {
+            if (stage > 0)
+                each([&](int k, int m, int i) {
+                    const double2 z = esm[cur + i];
+                    esm[cur + i] = make_double2(-W(0, k, m) * div_pow2_or_rn(z.x, Md, rM, pow2),
+                                                qc ? -W(1, k, m) * div_pow2_or_rn(z.y, Md, rM, pow2) : 0.0);
+                });
+            forward();
+            each([&](int k, int m, int i) {
+                const double2 z = esm[cur + i];
+                double2 r;
+                if (stage == 0) {
+                    Nv(k, m) = z;
+                    r = lin2(T(1, k, m), V(k, m), T(2, k, m), z);
+                    A(k, m) = r;
+                } else if (stage == 1) {
+                    S(k, m) = z;
+                    r = lin2(T(1, k, m), V(k, m), T(2, k, m), z);
+                } else if (stage == 2) {
+                    const double2 nv = Nv(k, m), na = S(k, m);
+                    S(k, m) = make_double2(na.x + z.x, na.y + z.y);
+                    r = lin2(T(1, k, m), A(k, m), T(2, k, m), make_double2(2.0 * z.x - nv.x, 2.0 * z.y - nv.y));
+                } else {
+                    const double2 v = V(k, m), nv = Nv(k, m), s = S(k, m);
+                    const double e = T(0, k, m), g1 = T(3, k, m), c2 = 2.0 * T(4, k, m), g3 = T(5, k, m);
+                    r = make_double2(e * v.x + g1 * nv.x + c2 * s.x + g3 * z.x, e * v.y + g1 * nv.y + c2 * s.y + g3 * z.y);
+                    V(k, m) = r;
+                }
+                esm[cur + i] = r;
+            });
+            inverse();
+        }
+        double *of = a.hf + (long)(t + 1) * M, *oc = a.hc ? a.hc + (long)(t + 1) * M : nullptr;
+        each([&](int k, int m, int i) {
+            const double2 z = esm[cur + i];
+            const double2 x = make_double2(div_pow2_or_rn(z.x, Md, rM, pow2), div_pow2_or_rn(z.y, Md, rM, pow2));
+            of[m] = x.x;
+            if (oc) oc[m] = x.y;
+            if constexpr (REGS) q[k] = x;
+        });
+    }
+}
+
+size_t small_smem(int Lx, int Ly) { return sizeof(double2) * ((size_t)Lx + Ly + 2 * (size_t)Lx * (Ly | 1)); }
+
+bool small_grid(int Lx, int Ly, int Lz) {
+    return Lz == 1 && Lx > 1 && (long)Lx * Ly <= kSmallPoints && small_smem(Lx, Ly) <= 200 * 1024;
+}
+
+// f(kernel, threads) of the grid's kernel
+template <class F>
+void small_kernel(long M, F f) {
+    if (M <= 128) f(etd_small_kernel<64, 2>, 64);
+    else if (M <= 1024) f(etd_small_kernel<256, 4>, 256);
+    else if (M <= 2048) f(etd_small_kernel<512, 4>, 512);
+    else f(etd_small_kernel<512, 8>, 512);
+}
+
 }  // namespace
 
 // Etdrk4_PBC's tables (Etdrk4_PBC.cc:14-24, :43-99): E = exp(ds L),
@@ -142,8 +357,19 @@ void PairChain::set_tables_etd(const std::vector<double>& k2, double ds, int Mc)
         tab[4 * M + m] = ds * (s2 / Mc);
         tab[5 * M + m] = ds * (s3 / Mc);
     }
+    if (small_etd()) {
+        small_kernel(M_, [](auto kernel, int) {
+            PS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        });
+    }
     etdtab_.alloc(tab.size());
     PS_CUDA(cudaMemcpy(etdtab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+}
+
+// PS_B200_LINE_PASSES=1 keeps the line passes
+bool PairChain::small_etd() const {
+    const char* force = getenv("PS_B200_LINE_PASSES");
+    return scheme_ == SCHEME_ETDRK4 && small_grid(Lx_, Ly_, Lz_) && !(force && force[0] == '1');
 }
 
 // forward (MODE_FWD) or inverse (MODE_INV, unnormalised) transform of one
@@ -171,6 +397,26 @@ void PairChain::enqueue_etd(double* hf, double* hc, int nsteps, const LaneFactor
     f.T = T;
     f.V = etd_.c(); f.Nv = f.V + M; f.A = f.V + 2 * M; f.Na = f.V + 3 * M; f.Nb = f.V + 4 * M;
     f.E = etdtab_.p; f.E2 = f.E + M; f.Q = f.E + 2 * M; f.f1 = f.E + 3 * M; f.f2 = f.E + 4 * M; f.f3 = f.E + 5 * M;
+    if (small_etd()) {
+        EtdSmall a{};
+        a.hf = hf;
+        a.hc = c_in_fixed ? nullptr : hc;   // a fixed lane c is zero (UpdaterCtx)
+        for (int i = 0; i < 2; i++) {
+            a.wf[i] = lf.eF[i];
+            a.wc[i] = lc.eF[i];
+        }
+        a.swf = lf.switch_t; a.swc = lc.switch_t;
+        a.nsteps = nsteps; a.Lx = Lx_; a.Ly = Ly_;
+        a.E = f.E; a.E2 = f.E2; a.Q = f.Q; a.f1 = f.f1; a.f2 = f.f2; a.f3 = f.f3;
+        a.V = f.V; a.Nv = f.Nv; a.A = f.A; a.S = f.Na;
+        a.twx = twiddle_table(Lx_);
+        a.twy = Ly_ > 1 ? twiddle_table(Ly_) : nullptr;
+        small_kernel(M, [&](auto kernel, int threads) {
+            kernel<<<1, threads, small_smem(Lx_, Ly_), st>>>(a);
+        });
+        PS_CUDA(cudaGetLastError());
+        return;
+    }
     for (int t = 0; t < nsteps; t++) {
         const double* qf = hf + (long)t * M;
         const double* qc = c_in_fixed ? c_in_fixed : hc + (long)t * M;
