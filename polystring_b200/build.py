@@ -20,7 +20,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
          "--expt-relaxed-constexpr", "-I", os.path.join(HERE, "..", "include")]
 
-SOURCES = ["line_pass.cu", "real_sweep.cu", "plane_sweep.cu", "cluster_sweep.cu", "twiddles.cu", "field_kernels.cu", "anderson.cu", "engine.cu", "adjoint.cu", "adjoint_sweep.cu", "string_ab.cu", "capi.cu", "density_noalloc.cu", "autotune.cu", "grouped_pass.cu", "batch_ab.cu", "fp64_peak.cu", "etdrk4.cu", "model_abc.cu"]
+SOURCES = ["line_pass.cu", "real_sweep.cu", "plane_sweep.cu", "tile_sweep.cu", "cluster_sweep.cu", "twiddles.cu", "field_kernels.cu", "anderson.cu", "engine.cu", "adjoint.cu", "adjoint_sweep.cu", "string_ab.cu", "capi.cu", "density_noalloc.cu", "autotune.cu", "grouped_pass.cu", "batch_ab.cu", "fp64_peak.cu", "etdrk4.cu", "model_abc.cu"]
 
 
 def _headers():

@@ -231,6 +231,8 @@ void stress_launch(const StressArgs& a, cudaStream_t st) {
 // the grid has no sweep or the device has no room: the line passes serve then.
 bool ModelAB::sweep_adjoint(bool grad) {
     if (!real_ || p_.dim < 2) return false;
+    // the stress keeps an axis's operator in shared memory: 36 KB at 128 points, 250 KB at 352
+    if (!grad && (p_.Lx > 128 || p_.Ly > 128 || p_.Lz > 128)) return false;
     const size_t n = (size_t)Ns_ * M_;
     try {
         for (DevBuf* b : {&kept_[0], &kept_[1], &kept_[2], &kept_[3]})

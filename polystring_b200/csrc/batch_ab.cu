@@ -122,14 +122,20 @@ RealProblem BatchAB::sweep_descriptor(int k) const {
     return k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
 }
 
-// one launch of the solves ks, per[i] CTAs a chain (3D)
+bool BatchAB::plane(int k) const {
+    const RealProblem p = sweep_descriptor(k);
+    return p.Lz == 1 && plane_sweep_supported(p.Lx, p.Ly);
+}
+
+// one launch of the solves ks, per[i] CTAs a chain (not for 2D up to 64 x 64)
 void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per) {
     chunks_.emplace_back();
     SweepChunk& c = chunks_.back();
     c.n = (int)ks.size();
     std::vector<RealProblem> d;
     for (int k : ks) d.push_back(sweep_descriptor(k));
-    c.plane = d[0].Lz == 1;
+    c.plane = plane(ks[0]);
+    c.tile = !c.plane && d[0].Lz == 1;
     if (c.plane) {
         for (const RealProblem& p : d) c.pairs = std::max(c.pairs, plane_sweep_pairs(p.Lx, p.Ly));
         for (const RealProblem& p : d) c.smem = std::max(c.smem, plane_sweep_smem(p, c.pairs));
@@ -139,9 +145,10 @@ void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per)
             d[i].bar = c.bar + 32 * (size_t)i;
             d[i].cta0 = c.grid;
             d[i].ncta = per[i];
+            d[i].split = c.tile && tile_sweep_split(d[i], per[i]);
             c.grid += 2 * per[i];
-            c.smem = std::max(c.smem, real_sweep_smem(d[i]));
-            c.wide = c.wide || real_sweep_wide(d[i]);
+            c.smem = std::max(c.smem, c.tile ? tile_sweep_smem(d[i]) : real_sweep_smem(d[i]));
+            c.wide = c.wide || (!c.tile && real_sweep_wide(d[i]));
         }
     }
     PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
@@ -149,12 +156,30 @@ void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per)
 }
 
 void BatchAB::build_sweeps(const std::vector<int>& members) {
-    // 2D solves: a CTA a chain, independent of each other, one launch
-    std::vector<int> planes, ks;
-    for (int k : members) (sweep_descriptor(k).Lz == 1 ? planes : ks).push_back(k);
+    // 2D solves up to 64 x 64: a CTA a chain, independent of each other, one launch
+    std::vector<int> planes, tiles, ks;
+    for (int k : members) (plane(k) ? planes : sweep_descriptor(k).Lz == 1 ? tiles : ks).push_back(k);
     auto longer = [&](int a, int b) { return Ns_of(a) > Ns_of(b); };
     std::stable_sort(planes.begin(), planes.end(), longer);
     if (!planes.empty()) add_chunk(planes, {});
+    // larger 2D solves: as many to a launch as have room with a CTA a tile (128^2: four)
+    std::stable_sort(tiles.begin(), tiles.end(), longer);
+    for (size_t i = 0; i < tiles.size();) {
+        std::vector<int> part, per;
+        size_t smem = 0;
+        int ctas = 0;
+        for (; i < tiles.size(); i++) {
+            const RealProblem p = sweep_descriptor(tiles[i]);
+            const int n = tile_sweep_tasks(p.Lx, p.Ly);
+            smem = std::max(smem, tile_sweep_smem(p));
+            if (!part.empty() && ctas + 2 * n > tile_sweep_resident(smem)) break;
+            part.push_back(tiles[i]);
+            per.push_back(n);
+            ctas += 2 * n;
+        }
+        if (part.size() == 1) own_.push_back(part[0]);
+        else add_chunk(part, per);
+    }
     // 3D solves: a launch lasts its longest solve's Ns steps.  A step of a solve
     // alone takes about 5 us for its two barriers and phases' latencies and
     // 24 ps a point and chain (7.4, 12.4, 17.6 us at 32^3, 48^3, 64^3); one of a
@@ -290,7 +315,8 @@ void BatchAB::enqueue_iteration() {
             plane_sweep_launch_many(c.dev, c.n, c.pairs, c.smem, st_);
         } else {
             PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-            real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
+            if (c.tile) tile_sweep_launch_many(c.dev, c.n, c.smem, c.grid, st_);
+            else real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
         }
         launches++;
     }

@@ -459,7 +459,7 @@ void launch(const RealProblem& p, const RealProblem* d, int n, size_t smem, bool
 
 }  // namespace
 
-std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, bool parts, int fo[3]) {
+std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, int fragments, int fo[3]) {
     std::vector<double> out;
     for (int a = 0; a < 3; a++) {
         fo[a] = -1;
@@ -474,7 +474,7 @@ std::vector<double> real_operator_tables(const int n[3], const double k[3], doub
                 const int r = i < n[a] / 2 + 1 ? i : n[a] - i;
                 L[i] = exp(h * (k[a] * r * r));
             }
-            if (parts) real_parts(n[a], L, out);
+            if (n[a] > fragments) real_parts(n[a], L, out);
             else real_fragments(n[a], L, out);
         }
     }
@@ -540,7 +540,7 @@ void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool one, 
 // ---------------------------------------------------------------------------
 bool RealSweep::supported(int Lx, int Ly, int Lz) {
     if (Ly == 1 && Lz == 1) return line_sweep_supported(Lx);
-    if (Lz == 1) return plane_sweep_supported(Lx, Ly);
+    if (Lz == 1) return plane_sweep_supported(Lx, Ly) || tile_sweep_supported(Lx, Ly);
     return real_sweep_supported(Lx, Ly, Lz);
 }
 
@@ -550,13 +550,22 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     const size_t M = (size_t)n[0] * n[1] * n[2];
     variant_ = 0;
     ncta_ = 0;
-    const std::vector<double> f = real_operator_tables(n, k, ds, dim_ == 1, fo_);
+    const bool plane = dim_ == 2 && plane_sweep_supported(n[0], n[1]);
+    // a single solve's chains in tiles over many CTAs where that is faster than a CTA
+    // a chain (us a step, tiles against one CTA: RQM4 64^2 5.9 / 9.1, 48 x 64 5.8 / 6.9,
+    // 48^2 5.7 / 5.4, 32^2 5.1 / 2.3; OS2 64^2 4.7 / 5.1, 48 x 64 4.7 / 3.9)
+    tile_ = dim_ == 2 && (!plane || n[0] * n[1] >= (os2 ? 64 * 64 : 48 * 64));
+    const std::vector<double> f = real_operator_tables(n, k, ds, dim_ == 1 ? 0 : dim_ == 2 ? tile_sweep_fragments() : 1 << 30, fo_);
     nfrag_ = (int)f.size();
     if (dim_ == 3) {
         ncta_ = std::max(1, std::min(prepare_kernels() / nl, real_sweep_tasks(n[0], n[1], n[2])));
         PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
-    } else if (dim_ == 2) {
-        plane_sweep_prepare();
+    }
+    if (plane) plane_sweep_prepare();
+    if (tile_) {
+        const int most = tile_sweep_resident(tile_sweep_smem(problem(nullptr, 0)));
+        ncta_ = std::max(1, std::min(most / nl, tile_sweep_tasks(n[0], n[1])));
+        PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
     }
     PS_CUDA(cudaMalloc(&frag_, sizeof(double) * f.size()));
     PS_CUDA(cudaMemcpy(frag_, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
@@ -573,7 +582,7 @@ RealSweep::~RealSweep() {
 RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
     const size_t M = (size_t)n_[0] * n_[1] * n_[2];
     RealProblem p{};
-    for (int i = 0; i < nl_; i++) p.lane[i] = lanes[i];
+    if (lanes) std::copy(lanes, lanes + nl_, p.lane);
     p.W = work_;
     p.Z = work_ + nl_ * M;
     p.frag = frag_;
@@ -591,8 +600,9 @@ RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
 
 void RealSweep::enqueue(const RealProblem& p, cudaStream_t st) const {
     if (dim_ == 1) return line_sweep_launch(p, st);
-    if (dim_ == 2) return plane_sweep_launch(p, st);
+    if (dim_ == 2 && !tile_) return plane_sweep_launch(p, st);
     PS_CUDA(cudaMemsetAsync(bar_, 0, 32 * sizeof(unsigned), st));
+    if (tile_) return tile_sweep_launch(p, ncta_, st);
     real_sweep_launch(p, ncta_, st);
 }
 

@@ -1,5 +1,6 @@
 // real_sweep.h -- propagator sweeps built on real line operators
-// (real_line.cuh): 3D grids in real_sweep.cu, 1D and 2D grids in plane_sweep.cu.
+// (real_line.cuh): 3D grids in real_sweep.cu, 1D grids and 2D grids of up to
+// 64 x 64 points in plane_sweep.cu, larger 2D grids in tile_sweep.cu.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -29,7 +30,7 @@ struct RealLane {
 struct RealProblem {
     RealLane lane[2];
     double *W, *Z;        // work fields, nl x M each
-    const double* frag;   // the axes' operators (full step, half step): B fragments (2D, 3D) or parts (1D)
+    const double* frag;   // the axes' operators (full step, half step): B fragments, or parts (1D; 2D axes past 64)
     int fo[3], nfrag;     // where each axis's start (axes of equal length and spacing share), doubles in all
     unsigned* bar;        // barrier counters (one a chain, 16 words apart), zeroed before the launch
     int* err;             // nonzero after a barrier timeout
@@ -37,13 +38,15 @@ struct RealProblem {
     int os2;              // second-order splitting: full steps only
     int xcols;            // columns of an x-pass task (a multiple of 8)
     int rkeep, xkeep;     // factors kept in shared memory: of the rows, of that many x-pass tasks a warp
+    int split;            // long rows in parts (tile_sweep.cu)
     int cta0, ncta;       // the solve's first CTA in a shared launch, CTAs of each chain
 };
 
 // the axes' operators of an orthogonal cell, exp(h k r^2) per axis for h = ds and
 // ds / 2, k = -(wave number)^2 at index 1; fo[a]: where axis a's start (axes
-// of the same length and k share theirs)
-std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, bool parts, int fo[3]);
+// of the same length and k share theirs); fragments of axes up to that many points,
+// parts of longer ones
+std::vector<double> real_operator_tables(const int n[3], const double k[3], double ds, int fragments, int fo[3]);
 
 // whether a 3D grid has this sweep
 bool real_sweep_supported(int Lx, int Ly, int Lz);
@@ -72,6 +75,17 @@ void plane_sweep_launch(const RealProblem& p, cudaStream_t st);
 int plane_sweep_pairs(int Lx, int Ly);
 size_t plane_sweep_smem(const RealProblem& p, int pairs);
 void plane_sweep_launch_many(const RealProblem* d, int n, int pairs, size_t smem, cudaStream_t st);
+// 2D grids, CTAs in tiles of lines; longest axis whose operators are fragments
+int tile_sweep_fragments();
+bool tile_sweep_supported(int Lx, int Ly);
+// CTAs one chain can keep busy, shared memory of a solve, CTAs resident at once
+int tile_sweep_tasks(int Lx, int Ly);
+bool tile_sweep_split(const RealProblem& p, int ncta);   // RealProblem::split with so many CTAs a chain
+size_t tile_sweep_smem(const RealProblem& p);
+int tile_sweep_resident(size_t smem);
+// ncta CTAs a chain; n solves described in device memory, grid CTAs in all
+void tile_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
+void tile_sweep_launch_many(const RealProblem* d, int n, size_t smem, int grid, cudaStream_t st);
 // 1D grids
 bool line_sweep_supported(int Lx);
 void line_sweep_launch(const RealProblem& p, cudaStream_t st);
@@ -93,10 +107,12 @@ public:
     // PS_B200_SWEEP_VARIANT=v forces variant v)
     void tune(const RealProblem& p, cudaStream_t st);
     void enqueue(const RealProblem& p, cudaStream_t st) const;
+    bool tiled() const { return tile_; }   // a 2D grid past 64 x 64
     int error(cudaStream_t st) const;   // barrier error flag (synchronises)
 
 private:
     int n_[3], dim_, nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
+    bool tile_ = false;
     double *work_ = nullptr, *frag_ = nullptr;
     unsigned* bar_ = nullptr;   // 32 words, then the error flag
 };
