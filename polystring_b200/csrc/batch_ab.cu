@@ -12,8 +12,8 @@
 // Ns, so the active ones are a prefix), each CTA running the pass body of its
 // own solve (grouped_pass.cu).  Members are grouped by the number of grid
 // axes longer than one (2 or 3), which fixes the pass sequence of a step.
-// Solves on grids with a persistent sweep take it instead: 2D solves in one
-// launch, a CTA a chain (plane_sweep.cu); 3D solves in launches that a cost
+// Solves on grids with a persistent sweep take it instead: 2D solves in a
+// launch of a CTA (plane_sweep.cu) or a cluster a chain (tile_sweep.cu); 3D solves in launches that a cost
 // model picks, sharing the SMs or alone (real_sweep.cu).  One batch iteration --
 // all propagators, then every member's Q, densities and field update -- is
 // captured once as a CUDA graph and replayed.
@@ -122,33 +122,34 @@ RealProblem BatchAB::sweep_descriptor(int k) const {
     return k < (int)m_.size() ? m_[k]->sweep_descriptor() : t_[k - m_.size()]->sweep_descriptor();
 }
 
-bool BatchAB::plane(int k) const {
-    const RealProblem p = sweep_descriptor(k);
-    return p.Lz == 1 && plane_sweep_supported(p.Lx, p.Ly);
+const RealSweep* BatchAB::sweep_of(int k) const {
+    return k < (int)m_.size() ? m_[k]->sweep() : t_[k - m_.size()]->sweep();
 }
 
-// one launch of the solves ks, per[i] CTAs a chain (not for 2D up to 64 x 64)
-void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per) {
+// one launch of the solves ks: 3D with per[i] CTAs a chain, 2D with a cluster or
+// (cluster = 0) a CTA a chain
+void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per, int cluster) {
     chunks_.emplace_back();
     SweepChunk& c = chunks_.back();
     c.n = (int)ks.size();
+    c.cluster = cluster;
     std::vector<RealProblem> d;
     for (int k : ks) d.push_back(sweep_descriptor(k));
-    c.plane = plane(ks[0]);
-    c.tile = !c.plane && d[0].Lz == 1;
+    c.plane = per.empty() && !cluster;
     if (c.plane) {
         for (const RealProblem& p : d) c.pairs = std::max(c.pairs, plane_sweep_pairs(p.Lx, p.Ly));
         for (const RealProblem& p : d) c.smem = std::max(c.smem, plane_sweep_smem(p, c.pairs));
+    } else if (cluster) {
+        for (const RealProblem& p : d) c.smem = std::max(c.smem, tile_sweep_smem(p));
     } else {
         PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * d.size()));
         for (int i = 0; i < c.n; i++) {
             d[i].bar = c.bar + 32 * (size_t)i;
             d[i].cta0 = c.grid;
             d[i].ncta = per[i];
-            d[i].split = c.tile && tile_sweep_split(d[i], per[i]);
             c.grid += 2 * per[i];
-            c.smem = std::max(c.smem, c.tile ? tile_sweep_smem(d[i]) : real_sweep_smem(d[i]));
-            c.wide = c.wide || (!c.tile && real_sweep_wide(d[i]));
+            c.smem = std::max(c.smem, real_sweep_smem(d[i]));
+            c.wide = c.wide || real_sweep_wide(d[i]);
         }
     }
     PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
@@ -156,29 +157,34 @@ void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per)
 }
 
 void BatchAB::build_sweeps(const std::vector<int>& members) {
-    // 2D solves up to 64 x 64: a CTA a chain, independent of each other, one launch
-    std::vector<int> planes, tiles, ks;
-    for (int k : members) (plane(k) ? planes : sweep_descriptor(k).Lz == 1 ? tiles : ks).push_back(k);
+    // 2D solves in one launch for each form.  In tiles, a cluster a chain, where a
+    // single solve takes that form; but solves up to 64 x 64 a CTA a chain when they
+    // are more than have clusters at once (64^2: 4.4 us a step for up to eight solves,
+    // 9.1 for up to 74)
+    std::vector<int> planes, tiles[2], ks;
     auto longer = [&](int a, int b) { return Ns_of(a) > Ns_of(b); };
-    std::stable_sort(planes.begin(), planes.end(), longer);
-    if (!planes.empty()) add_chunk(planes, {});
-    // larger 2D solves: as many to a launch as have room with a CTA a tile (128^2: four)
-    std::stable_sort(tiles.begin(), tiles.end(), longer);
-    for (size_t i = 0; i < tiles.size();) {
-        std::vector<int> part, per;
-        size_t smem = 0;
-        int ctas = 0;
-        for (; i < tiles.size(); i++) {
-            const RealProblem p = sweep_descriptor(tiles[i]);
-            const int n = tile_sweep_tasks(p.Lx, p.Ly);
-            smem = std::max(smem, tile_sweep_smem(p));
-            if (!part.empty() && ctas + 2 * n > tile_sweep_resident(smem)) break;
-            part.push_back(tiles[i]);
-            per.push_back(n);
-            ctas += 2 * n;
-        }
-        if (part.size() == 1) own_.push_back(part[0]);
-        else add_chunk(part, per);
+    for (int k : members) {
+        const RealProblem p = sweep_descriptor(k);
+        const RealSweep& s = *sweep_of(k);
+        if (p.Lz > 1) ks.push_back(k);
+        else if (s.cluster()) tiles[s.cluster() > 8].push_back(k);
+        else if (s.tiled()) own_.push_back(k);   // no room for clusters on this device
+        else planes.push_back(k);
+    }
+    std::vector<int> small;
+    for (int k : tiles[0]) {
+        const RealProblem p = sweep_descriptor(k);
+        if (plane_sweep_supported(p.Lx, p.Ly)) small.push_back(k);
+    }
+    size_t most_smem = 0;
+    for (int k : small) most_smem = std::max(most_smem, tile_sweep_smem(sweep_descriptor(k)));
+    if (!small.empty() && 2 * (int)small.size() > tile_cluster_resident(8, most_smem)) {
+        planes.insert(planes.end(), small.begin(), small.end());
+        for (int k : small) tiles[0].erase(std::find(tiles[0].begin(), tiles[0].end(), k));
+    }
+    for (std::vector<int>* v : {&planes, &tiles[0], &tiles[1]}) {
+        std::stable_sort(v->begin(), v->end(), longer);
+        if (!v->empty()) add_chunk(*v, {}, v == &planes ? 0 : v == &tiles[0] ? 8 : 16);
     }
     // 3D solves: a launch lasts its longest solve's Ns steps.  A step of a solve
     // alone takes about 5 us for its two barriers and phases' latencies and
@@ -228,7 +234,7 @@ void BatchAB::build_sweeps(const std::vector<int>& members) {
             const RealProblem p = sweep_descriptor(k);
             per.push_back(std::min(real_sweep_tasks(p.Lx, p.Ly, p.Lz), 1 + (int)(spare * (points_of(k) / points))));
         }
-        add_chunk(part, per);
+        add_chunk(part, per, 0);
     }
 }
 
@@ -313,10 +319,11 @@ void BatchAB::enqueue_iteration() {
     for (const SweepChunk& c : chunks_) {
         if (c.plane) {
             plane_sweep_launch_many(c.dev, c.n, c.pairs, c.smem, st_);
+        } else if (c.cluster) {
+            tile_cluster_launch_many(c.dev, c.n, c.cluster, c.smem, st_);
         } else {
             PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-            if (c.tile) tile_sweep_launch_many(c.dev, c.n, c.smem, c.grid, st_);
-            else real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
+            real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
         }
         launches++;
     }

@@ -41,10 +41,11 @@ private:
         size_t smem[9] = {};
     };
     // solves that share a sweep launch: their descriptors on the device, and
-    // 32 barrier words each (3D and large 2D)
+    // 32 barrier words each (3D)
     struct SweepChunk {
         int n = 0, grid = 0, pairs = 0;
-        bool plane = false, tile = false, wide = false;
+        int cluster = 0;
+        bool plane = false, wide = false;
         size_t smem = 0;
         RealProblem* dev = nullptr;
         unsigned* bar = nullptr;
@@ -55,8 +56,8 @@ private:
     int Ns_of(int k) const;
     double points_of(int k) const;
     RealProblem sweep_descriptor(int k) const;
-    bool plane(int k) const;            // a 2D solve with a CTA a chain
-    void add_chunk(const std::vector<int>& ks, const std::vector<int>& per);
+    const RealSweep* sweep_of(int k) const;
+    void add_chunk(const std::vector<int>& ks, const std::vector<int>& per, int cluster);
     void build_sweeps(const std::vector<int>& members);
     void release();
     void enqueue_iteration();

@@ -468,8 +468,8 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     launch_fill(hf_.p, M_, 1.0, st_);
     launch_fill(hc_.p, M_, 1.0, st_);
     launch_fill(yita_.p, M_, 0.0, st_);
-    // (line passes also serve the adjoint where its sweep does not)
-    if ((!real_ || real_->tiled()) && !batch_member) chain_->autotune(st_);
+    // the line passes of larger 2D grids also serve where the adjoint's sweep does not
+    if ((!real_ || (p.dim == 2 && std::max(p.Lx, p.Ly) > 64)) && !batch_member) chain_->autotune(st_);
     if (real_ && !batch_member) {
         // finite data for the timed sweeps (set_fields overwrites the factors)
         for (double* f : {eFA_.p, eHA_.p, eFB_.p, eHB_.p}) launch_fill(f, M_, 1.0, st_);

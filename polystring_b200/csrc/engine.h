@@ -186,7 +186,8 @@ public:
     long iterations() const { return iter_; }
     int status();
     const ModelABParams& params() const { return p_; }
-    bool persistent_sweep() const { return real_ != nullptr; }   // real_sweep.cu
+    bool persistent_sweep() const { return real_ != nullptr; }
+    const RealSweep* sweep() const { return real_; }
     // the sweep's description of this solve (its own work fields, barrier
     // words and error flag)
     RealProblem sweep_descriptor() const;
@@ -302,6 +303,7 @@ public:
     int launches_post() const { return 2 + 3 + (p_.scft == 1 ? 4 : 1); }
     // the persistent sweep with three factor sets
     bool persistent_sweep() const { return real_ != nullptr; }
+    const RealSweep* sweep() const { return real_; }
     RealProblem sweep_descriptor() const;
     const ModelABCParams& params() const { return p_; }
 

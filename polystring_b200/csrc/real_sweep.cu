@@ -552,9 +552,9 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     ncta_ = 0;
     const bool plane = dim_ == 2 && plane_sweep_supported(n[0], n[1]);
     // a single solve's chains in tiles over many CTAs where that is faster than a CTA
-    // a chain (us a step, tiles against one CTA: RQM4 64^2 5.9 / 9.1, 48 x 64 5.8 / 6.9,
-    // 48^2 5.7 / 5.4, 32^2 5.1 / 2.3; OS2 64^2 4.7 / 5.1, 48 x 64 4.7 / 3.9)
-    tile_ = dim_ == 2 && (!plane || n[0] * n[1] >= (os2 ? 64 * 64 : 48 * 64));
+    // a chain (us a step, tiles against one CTA: RQM4 64^2 4.4 / 9.1, 48^2 4.2 / 5.4,
+    // 32 x 64 3.8 / 4.3, 32^2 3.5 / 2.3; OS2 64^2 3.2 / 5.1, 48^2 3.1 / 3.1, 32 x 64 3.0 / 2.5)
+    tile_ = dim_ == 2 && (!plane || n[0] * n[1] >= (os2 ? 48 * 64 : 32 * 64));
     const std::vector<double> f = real_operator_tables(n, k, ds, dim_ == 1 ? 0 : dim_ == 2 ? tile_sweep_fragments() : 1 << 30, fo_);
     nfrag_ = (int)f.size();
     if (dim_ == 3) {
@@ -563,8 +563,10 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     }
     if (plane) plane_sweep_prepare();
     if (tile_) {
-        const int most = tile_sweep_resident(tile_sweep_smem(problem(nullptr, 0)));
-        ncta_ = std::max(1, std::min(most / nl, tile_sweep_tasks(n[0], n[1])));
+        const size_t smem = tile_sweep_smem(problem(nullptr, 0));
+        cluster_ = tile_cluster_size(n[0], n[1]);
+        if (cluster_ && tile_cluster_resident(cluster_, smem) < 1) cluster_ = 0;
+        if (!cluster_) ncta_ = std::max(1, std::min(tile_sweep_resident(smem) / nl, tile_sweep_tasks(n[0], n[1])));
         PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
     }
     PS_CUDA(cudaMalloc(&frag_, sizeof(double) * f.size()));
@@ -601,6 +603,7 @@ RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
 void RealSweep::enqueue(const RealProblem& p, cudaStream_t st) const {
     if (dim_ == 1) return line_sweep_launch(p, st);
     if (dim_ == 2 && !tile_) return plane_sweep_launch(p, st);
+    if (cluster_) return tile_cluster_launch(p, cluster_, st);
     PS_CUDA(cudaMemsetAsync(bar_, 0, 32 * sizeof(unsigned), st));
     if (tile_) return tile_sweep_launch(p, ncta_, st);
     real_sweep_launch(p, ncta_, st);

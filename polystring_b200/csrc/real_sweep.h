@@ -75,17 +75,26 @@ void plane_sweep_launch(const RealProblem& p, cudaStream_t st);
 int plane_sweep_pairs(int Lx, int Ly);
 size_t plane_sweep_smem(const RealProblem& p, int pairs);
 void plane_sweep_launch_many(const RealProblem* d, int n, int pairs, size_t smem, cudaStream_t st);
-// 2D grids, CTAs in tiles of lines; longest axis whose operators are fragments
+// 2D grids in tiles of lines; longest axis whose operators are fragments
 int tile_sweep_fragments();
 bool tile_sweep_supported(int Lx, int Ly);
-// CTAs one chain can keep busy, shared memory of a solve, CTAs resident at once
+// CTAs one chain can keep busy, shared memory of a solve
 int tile_sweep_tasks(int Lx, int Ly);
-bool tile_sweep_split(const RealProblem& p, int ncta);   // RealProblem::split with so many CTAs a chain
 size_t tile_sweep_smem(const RealProblem& p);
+// over the whole grid: CTAs resident at once; ncta CTAs a chain
 int tile_sweep_resident(size_t smem);
-// ncta CTAs a chain; n solves described in device memory, grid CTAs in all
 void tile_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
-void tile_sweep_launch_many(const RealProblem* d, int n, size_t smem, int grid, cudaStream_t st);
+// a cluster a chain: its size for a grid (0: none) and the clusters resident at
+// once; a solve, or n solves of two chains described in device memory
+int tile_cluster_size(int Lx, int Ly);
+int tile_cluster_resident(int cluster, size_t smem);
+void tile_cluster_launch(const RealProblem& p, int cluster, cudaStream_t st);
+void tile_cluster_launch_many(const RealProblem* d, int n, int cluster, size_t smem, cudaStream_t st);
+// n solves of two chains on one 2D grid with axes up to 128 points (the images of a
+// string), a cluster each; prepare notes the clusters resident at once
+bool tile_string_supported(int Lx, int Ly);
+void tile_string_prepare(const RealProblem& p, int n);
+void tile_string_launch(const RealProblem* d, int n, size_t smem, cudaStream_t st);
 // 1D grids
 bool line_sweep_supported(int Lx);
 void line_sweep_launch(const RealProblem& p, cudaStream_t st);
@@ -107,12 +116,14 @@ public:
     // PS_B200_SWEEP_VARIANT=v forces variant v)
     void tune(const RealProblem& p, cudaStream_t st);
     void enqueue(const RealProblem& p, cudaStream_t st) const;
-    bool tiled() const { return tile_; }   // a 2D grid past 64 x 64
+    bool tiled() const { return tile_; }   // 2D, the chains in tiles of lines
+    int cluster() const { return cluster_; }
     int error(cudaStream_t st) const;   // barrier error flag (synchronises)
 
 private:
     int n_[3], dim_, nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
     bool tile_ = false;
+    int cluster_ = 0;   // CTAs of a chain's cluster (0: chains over the grid)
     double *work_ = nullptr, *frag_ = nullptr;
     unsigned* bar_ = nullptr;   // 32 words, then the error flag
 };

@@ -199,7 +199,8 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
     const char* force = getenv("PS_B200_LINE_PASSES");
     const bool lines = force && force[0] == '1';
     if (!lines && p.Ly > 1 && p.Lz == 1 && (p.mde == 0 || cell_separable(p_.cell)) &&
-        plane_sweep_supported(p.Lx, p.Ly)) {
+        (plane_sweep_supported(p.Lx, p.Ly) ||
+         (tile_string_supported(p.Lx, p.Ly) && !(p.mde == 0 && cluster_sweep_supported(p.Lx, p.Ly, p.Lz))))) {
         const int n[3] = {p.Lx, p.Ly, 1};
         double k[3];
         axis_k2(p_.cell, k);
@@ -216,7 +217,8 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
         }
         chain_->set_tables(L1, L2);
         // 128^2: every image's propagators in one cluster-resident sweep per
-        // SCFT iteration
+        // SCFT iteration (with 40 images 43.5 us a contour step, in tiles 48.5: their
+        // fields pass through L2)
         if (!lines && cluster_sweep_supported(p.Lx, p.Ly, p.Lz)) {
             use_cluster_ = true;
             cluster_sweep_prepare(p.Lx, p.Ly, p.Lz, nloc_);
@@ -240,6 +242,8 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
     ends_.alloc(4 * (size_t)M_);
     if (real_) {
         const int never = 1 << 30;
+        tiled_ = !plane_sweep_supported(p.Lx, p.Ly);
+        if (tiled_) work_.alloc(4 * nM);
         std::vector<RealProblem> d;
         for (int b = 0; b < nloc_; b++) {
             double *hf = hf_.p + (size_t)b * (Ns_ + 1) * M_, *hc = hc_.p + (size_t)b * (Ns_ + 1) * M_;
@@ -247,7 +251,10 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
             const RealLane lanes[2] = {{hf, {fA, fB, fB}, {hA, hB, hB}, {LA_, never}},
                                        {hc, {fB, fA, fA}, {hB, hA, hA}, {LB_, never}}};
             d.push_back(real_->problem(lanes, Ns_));
+            d.back().Z = work_.p + 4 * b * M_;
+            d.back().W = d.back().Z + 2 * M_;
         }
+        if (tiled_) tile_string_prepare(d[0], nloc_);
         PS_CUDA(cudaMalloc(&images_, sizeof(RealProblem) * d.size()));
         PS_CUDA(cudaMemcpy(images_, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
     }
@@ -303,7 +310,9 @@ void StringAB::enqueue_scft_iteration() {
     if (real_) {
         const int pairs = plane_sweep_pairs(p_.Lx, p_.Ly);
         const RealLane none[2] = {};
-        plane_sweep_launch_many(images_, nloc_, pairs, plane_sweep_smem(real_->problem(none, Ns_), pairs), st_);
+        const RealProblem p = real_->problem(none, Ns_);
+        if (tiled_) tile_string_launch(images_, nloc_, tile_sweep_smem(p), st_);
+        else plane_sweep_launch_many(images_, nloc_, pairs, plane_sweep_smem(p, pairs), st_);
     } else if (use_cluster_) {
         SweepArgs a{};
         a.hf = hf_.p; a.hc = hc_.p;

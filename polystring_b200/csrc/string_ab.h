@@ -49,8 +49,11 @@ private:
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t giter_ = nullptr, grelax_ = nullptr, grepar_ = nullptr;
     DevBuf hf_, hc_, wa_, wb_, yita_, phiA_, phiB_, eFA_, eHA_, eFB_, eHB_, ends_, cA_, cB_, scal_, S_, partial_;
-    RealSweep* real_ = nullptr;          // one CTA a chain (plane_sweep.cu): operators, and
+    RealSweep* real_ = nullptr;          // operators of the images' persistent sweeps
     RealProblem* images_ = nullptr;      // the images' descriptions on the device
+    bool tiled_ = false;                 // an axis past 64 points: a cluster an image (tile_sweep.cu),
+                                         // else a CTA a chain (plane_sweep.cu)
+    DevBuf work_;                        // the tiled sweeps' fields
     // one thread-block cluster per image for the propagators (cluster_sweep.cu)
     bool use_cluster_ = false;
     DevBuf clK_;                         // per-axis exp(h k^2): x, y for h = ds, then ds / 2

@@ -22,6 +22,7 @@
 // where the fragments take 64 KB).  The arithmetic of a line does not depend on how tiles
 // are spread over CTAs.
 #include <algorithm>
+#include <cstdio>
 
 #include "engine.h"
 #include "ps_internal.h"
@@ -33,7 +34,8 @@ namespace ps {
 
 namespace {
 
-constexpr int kNT = 256;
+constexpr int kNT = 256;      // threads of a CTA of the grid form
+constexpr int kStringNT = 128;   // and of a string's clusters: three CTAs an SM
 constexpr long long kSpinLimit = 20000000;   // polls before a barrier gives up
 constexpr size_t kSmemLimit = 227 * 1024 - 1024;
 
@@ -64,6 +66,11 @@ __device__ __forceinline__ bool chain_barrier(unsigned* count, int* err, unsigne
     return stop == 0;
 }
 
+// barrier over the cluster's CTAs, with their writes to global memory
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ int lane_block(const RealLane& c, int t) { return t < c.sw[0] ? 0 : t < c.sw[1] ? 1 : 2; }
 
 // threadIdx.x, read anew where a phase starts: else the index arithmetic of every
@@ -80,14 +87,14 @@ __host__ __device__ constexpr int pitch_of(int n) { return (n & 7) == 4 ? n : n 
 
 constexpr int kFragments = 64;   // longest line whose operators are held as fragments
 
-template <int N>
+template <int N, int NT = kNT>
 struct Tile {
     using R = RealLine<N>;
     static constexpr int O = R::O, S = R::S, T = R::T;
     static constexpr int XP = pitch_of(4 * S), YP = pitch_of(8 * T);
     static constexpr int XF = 32 * XP, YF = 32 * YP;   // a field: [block][line][orbit]
     static constexpr int OP = N <= kFragments ? R::FRAG : 4 * R::PARTS;   // doubles of an operator
-    static constexpr int U = (8 * O + kNT - 1) / kNT;  // (line, orbit) items a thread
+    static constexpr int U = (8 * O + NT - 1) / NT;  // (line, orbit) items a thread
 };
 
 // folded values of field f, results of field f
@@ -123,10 +130,10 @@ __device__ __forceinline__ void take(const double* y, int g, int o, double (&v)[
 // unit a warp: the tiles share the folded values, and a tile's Toeplitz entries
 // are the next tile's two steps on, its Hankel entries two steps back.
 // TT output tiles from tile0 on (default: all).
-template <int N, int NF, int TT = Tile<N>::T>
+template <int N, int NT, int NF, int TT = Tile<N>::T>
 __device__ __forceinline__ void products(const Shared& m, const double* op0, const double* op1, int tile0 = 0) {
-    using Q = Tile<N>;
-    constexpr int P = Q::R::PARTS, S = Q::S, T = Q::T, UF = (kNT / 64) / NF;   // units a field and character
+    using Q = Tile<N, NT>;
+    constexpr int P = Q::R::PARTS, S = Q::S, T = Q::T, UF = (NT / 64) / NF;   // units a field and character
     constexpr int J = (TT + UF - 1) / UF, G = (TT + J - 1) / J;
     constexpr bool FULL = T % TT == 0 && TT % J == 0;   // no tile past the last one
     const int tid = thread_index(), warp = tid >> 5;
@@ -200,9 +207,9 @@ __device__ __forceinline__ double with_source(const RealLane& L, int t, long n, 
 }
 
 // columns of step t (N = Lx): tile of eight columns
-template <int N>
+template <int N, int NT>
 __device__ __forceinline__ void columns(const RealProblem& p, const double* op, const Shared& m, int ch, int tile, int t) {
-    using Q = Tile<N>;
+    using Q = Tile<N, NT>;
     using R = RealLine<N>;
     constexpr int HALF = Tile<N>::OP;
     const int tid = thread_index();
@@ -216,7 +223,7 @@ __device__ __forceinline__ void columns(const RealProblem& p, const double* op, 
     double f[Q::U][4];
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i & 7, o = i >> 3, y = 8 * tile + g;
+        const int i = tid + u * NT, g = i & 7, o = i >> 3, y = 8 * tile + g;
         if (o >= Q::O) continue;
         double z[4] = {0.0, 0.0, 0.0, 0.0}, w[4] = {0.0, 0.0, 0.0, 0.0};
         if (y < Ly) {
@@ -238,14 +245,14 @@ __device__ __forceinline__ void columns(const RealProblem& p, const double* op, 
         Shared w = m;
         w.x += m.xf;
         w.y += m.yf;
-        products<N, 1>(w, op, op);
+        products<N, NT, 1>(w, op, op);
     } else {
-        products<N, 2>(m, op + HALF, op);
+        products<N, NT, 2>(m, op + HALF, op);
     }
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i & 7, o = i >> 3, y = 8 * tile + g;
+        const int i = tid + u * NT, g = i & 7, o = i >> 3, y = 8 * tile + g;
         if (o >= Q::O) continue;
         double v[4];
         take<N>(m.y + m.yf, g, o, v);
@@ -267,11 +274,11 @@ __device__ __forceinline__ void columns(const RealProblem& p, const double* op, 
     }
     if (os2) return;
     __syncthreads();
-    products<N, 1>(m, op + HALF, op);
+    products<N, NT, 1>(m, op + HALF, op);
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i & 7, o = i >> 3, y = 8 * tile + g;
+        const int i = tid + u * NT, g = i & 7, o = i >> 3, y = 8 * tile + g;
         if (o >= Q::O || y >= Ly) continue;
         double v[4];
         take<N>(m.y, g, o, v);
@@ -282,9 +289,9 @@ __device__ __forceinline__ void columns(const RealProblem& p, const double* op, 
 
 // rows after step t (t < 0: the head) and the next step's inputs (N = Ly): tile
 // of eight rows
-template <int N>
+template <int N, int NT>
 __device__ __forceinline__ void rows(const RealProblem& p, const double* op, const Shared& m, int ch, int tile, int t) {
-    using Q = Tile<N>;
+    using Q = Tile<N, NT>;
     using R = RealLine<N>;
     constexpr int HALF = Tile<N>::OP;
     const int tid = thread_index();
@@ -300,7 +307,7 @@ __device__ __forceinline__ void rows(const RealProblem& p, const double* op, con
     double e[Q::U][4], q[Q::U][4], w[Q::U][4];
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
+        const int i = tid + u * NT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
         const bool on = i < 8 * Q::O && r < Lx;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -321,12 +328,12 @@ __device__ __forceinline__ void rows(const RealProblem& p, const double* op, con
     }
     if (t >= 0) {
         __syncthreads();
-        products<N, 1>(m, op + (os2 ? 0 : HALF), op);
+        products<N, NT, 1>(m, op + (os2 ? 0 : HALF), op);
         __syncthreads();
     }
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
+        const int i = tid + u * NT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
         if (i >= 8 * Q::O) continue;
         if (t >= 0) {
             double v[4];
@@ -379,11 +386,11 @@ __device__ __forceinline__ void rows(const RealProblem& p, const double* op, con
     }
     if (!next || os2) return;
     __syncthreads();
-    products<N, 2>(m, op + HALF, op);
+    products<N, NT, 2>(m, op + HALF, op);
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
+        const int i = tid + u * NT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
         if (i >= 8 * Q::O || r >= Lx) continue;
         double v[4];
         take<N>(m.y, g, o, v);
@@ -399,9 +406,9 @@ __device__ __forceinline__ void rows(const RealProblem& p, const double* op, con
 // rows, one of kParts parts of the output tiles), in two phases with a barrier
 // between.  q[t+1] of the part's orbits first.
 constexpr int kParts = 4;
-template <int N>
+template <int N, int NT>
 __device__ __forceinline__ void rows_first(const RealProblem& p, const double* op, const Shared& m, int ch, int task, int t) {
-    using Q = Tile<N>;
+    using Q = Tile<N, NT>;
     using R = RealLine<N>;
     constexpr int HALF = Tile<N>::OP, TT = (Q::T + kParts - 1) / kParts;
     const int tid = thread_index();
@@ -413,7 +420,7 @@ __device__ __forceinline__ void rows_first(const RealProblem& p, const double* o
     const double* const eb = L.eH[lane_block(L, t)];
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
+        const int i = tid + u * NT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
         if (i >= 8 * Q::O) continue;
         double v[4] = {0.0, 0.0, 0.0, 0.0};
         if (r < Lx)
@@ -422,7 +429,7 @@ __device__ __forceinline__ void rows_first(const RealProblem& p, const double* o
         put<N>(m.x, g, o, v);
     }
     // the part's orbits: thread (line, orbit)
-    static_assert(64 * TT <= kNT, "a thread takes one orbit of a part");
+    static_assert(64 * TT <= NT, "a thread takes one orbit of a part");
     const int g = tid / (8 * TT), o = 8 * tile0 + tid - g * 8 * TT, r = 8 * tile + g;
     const bool on = g < 8 && o < Q::O && r < Lx;
     const long row = (long)r * N;
@@ -434,7 +441,7 @@ __device__ __forceinline__ void rows_first(const RealProblem& p, const double* o
             w[k] = __ldcg(W + row + R::point(k, o));
         }
     __syncthreads();
-    products<N, 1, TT>(m, op + HALF, op, tile0);
+    products<N, NT, 1, TT>(m, op + HALF, op, tile0);
     __syncthreads();
     if (!on) return;
     double v[4];
@@ -449,9 +456,9 @@ __device__ __forceinline__ void rows_first(const RealProblem& p, const double* o
     }
 }
 // the next step's Z and W at the part's orbits
-template <int N>
+template <int N, int NT>
 __device__ __forceinline__ void rows_second(const RealProblem& p, const double* op, const Shared& m, int ch, int task, int t) {
-    using Q = Tile<N>;
+    using Q = Tile<N, NT>;
     using R = RealLine<N>;
     constexpr int HALF = Tile<N>::OP, TT = (Q::T + kParts - 1) / kParts;
     const int tid = thread_index();
@@ -462,7 +469,7 @@ __device__ __forceinline__ void rows_second(const RealProblem& p, const double* 
     const double* const eb = L.eH[lane_block(L, t + 1)];
 #pragma unroll
     for (int u = 0; u < Q::U; u++) {
-        const int i = tid + u * kNT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
+        const int i = tid + u * NT, g = i / Q::O, o = i - g * Q::O, r = 8 * tile + g;
         if (i >= 8 * Q::O) continue;
         double z[4] = {0.0, 0.0, 0.0, 0.0}, x[4] = {0.0, 0.0, 0.0, 0.0};
         if (r < Lx)
@@ -477,7 +484,7 @@ __device__ __forceinline__ void rows_second(const RealProblem& p, const double* 
         put<N>(m.x + m.xf, g, o, x);
     }
     __syncthreads();
-    products<N, 2, TT>(m, op + HALF, op, tile0);
+    products<N, NT, 2, TT>(m, op + HALF, op, tile0);
     __syncthreads();
     const int g = tid / (8 * TT), o = 8 * tile0 + tid - g * 8 * TT, r = 8 * tile + g;
     if (g >= 8 || o >= Q::O || r >= Lx) return;
@@ -500,71 +507,77 @@ __host__ __device__ __forceinline__ int x_doubles(int N) { return 32 * pitch_of(
 __host__ __device__ __forceinline__ int y_doubles(int N) { return 32 * pitch_of(8 * ((N / 4 + 7) / 8)); }
 __host__ __device__ __forceinline__ int most(int a, int b) { return a > b ? a : b; }
 
-__global__ void __launch_bounds__(kNT, 1) tile_sweep_kernel(const __grid_constant__ RealProblem one,
-                                                            const RealProblem* __restrict__ many, int n) {
+// MAX: longest line.  CTA b works on chain b / one.ncta, solve by solve (the solves
+// at `many`, or `one`).  GRID: one solve, a cooperative launch, a barrier in memory
+// for each chain.  Else clusters of one or two chains' CTAs with the hardware's
+// barrier, which wait for no other cluster: any number of them may queue.
+template <int NT, int PER_SM, int MAX, bool GRID>
+__global__ void __launch_bounds__(NT, PER_SM) tile_sweep_kernel(const __grid_constant__ RealProblem one,
+                                                                const RealProblem* __restrict__ many) {
     extern __shared__ __align__(16) double sm[];
     __shared__ RealProblem p;
-    __shared__ int which;
+    const int ncta = one.ncta, chain = (int)blockIdx.x / ncta, cta = (int)blockIdx.x - chain * ncta;
+    const int ch = chain % one.nl;
     if (many) {
-        for (int i = threadIdx.x; i < n; i += kNT) {
-            const int c = (int)blockIdx.x - many[i].cta0;
-            if (c >= 0 && c < many[i].ncta * many[i].nl) which = i;
-        }
-        __syncthreads();
         constexpr int W = sizeof(RealProblem) / 4;
-        for (int i = threadIdx.x; i < W; i += kNT)
-            reinterpret_cast<int*>(&p)[i] = reinterpret_cast<const int*>(many + which)[i];
+        for (int i = threadIdx.x; i < W; i += NT)
+            reinterpret_cast<int*>(&p)[i] = reinterpret_cast<const int*>(many + chain / one.nl)[i];
     } else if (threadIdx.x == 0) {
         p = one;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < p.nfrag; i += kNT) sm[i] = p.frag[i];
+    for (int i = threadIdx.x; i < p.nfrag; i += NT) sm[i] = p.frag[i];
     const double *opx = sm + p.fo[0], *opy = sm + p.fo[1];
     Shared m;
     m.xf = most(x_doubles(p.Lx), x_doubles(p.Ly));
     m.yf = most(y_doubles(p.Lx), y_doubles(p.Ly));
     m.x = sm + p.nfrag;
     m.y = m.x + 2 * m.xf;
-    const int ncta = p.ncta, ch = ((int)blockIdx.x - p.cta0) / ncta, cta = (int)blockIdx.x - p.cta0 - ch * ncta;
     const int rt = (p.Lx + 7) >> 3, ct = (p.Ly + 7) >> 3;
     unsigned* bar = p.bar + 16 * ch;
     unsigned target = 0;
+    auto barrier = [&]() {
+        if (!GRID) {
+            cluster_barrier();
+            return true;
+        }
+        target += ncta;
+        return chain_barrier(bar, p.err, target);
+    };
     for (int t = -1; t < p.Ns; t++) {
         if (t >= 0) {
             // orbits past the last one count as zero (the axes' layouts differ)
             if (p.Lx & 15) {
                 __syncthreads();
-                for (int i = threadIdx.x; i < 2 * m.xf; i += kNT) m.x[i] = 0.0;
+                for (int i = threadIdx.x; i < 2 * m.xf; i += NT) m.x[i] = 0.0;
             }
             for (int k = cta; k < ct; k += ncta) {
                 __syncthreads();
                 switch (p.Lx) {
-#define X(N) case N: columns<N>(p, opx, m, ch, k, t); break;
+#define X(N) case N: if constexpr (N <= MAX) columns<N, NT>(p, opx, m, ch, k, t); break;
                     TS_CASES(X)
 #undef X
                 }
             }
-            target += ncta;
-            if (!chain_barrier(bar, p.err, target)) return;
+            if (!barrier()) return;
         }
-        if (p.split) {
+        if (GRID && p.split) {
             if (t >= 0) {
                 for (int k = cta; k < kParts * rt; k += ncta) {
                     __syncthreads();
                     switch (p.Ly) {
-#define X(N) case N: rows_first<N>(p, opy, m, ch, k, t); break;
+#define X(N) case N: if constexpr (GRID) rows_first<N, NT>(p, opy, m, ch, k, t); break;
                         TS_LONG(X)
 #undef X
                     }
                 }
                 if (t + 1 == p.Ns) break;
-                target += ncta;
-                if (!chain_barrier(bar, p.err, target)) return;
+                if (!barrier()) return;
             }
             for (int k = cta; k < kParts * rt; k += ncta) {
                 __syncthreads();
                 switch (p.Ly) {
-#define X(N) case N: rows_second<N>(p, opy, m, ch, k, t); break;
+#define X(N) case N: if constexpr (GRID) rows_second<N, NT>(p, opy, m, ch, k, t); break;
                     TS_LONG(X)
 #undef X
                 }
@@ -572,20 +585,19 @@ __global__ void __launch_bounds__(kNT, 1) tile_sweep_kernel(const __grid_constan
         } else {
             if (p.Ly & 15) {
                 __syncthreads();
-                for (int i = threadIdx.x; i < 2 * m.xf; i += kNT) m.x[i] = 0.0;
+                for (int i = threadIdx.x; i < 2 * m.xf; i += NT) m.x[i] = 0.0;
             }
             for (int k = cta; k < rt; k += ncta) {
                 __syncthreads();
                 switch (p.Ly) {
-#define X(N) case N: rows<N>(p, opy, m, ch, k, t); break;
+#define X(N) case N: if constexpr (N <= MAX) rows<N, NT>(p, opy, m, ch, k, t); break;
                     TS_CASES(X)
 #undef X
                 }
             }
         }
         if (t + 1 < p.Ns) {
-            target += ncta;
-            if (!chain_barrier(bar, p.err, target)) return;
+            if (!barrier()) return;
         }
     }
 }
@@ -605,18 +617,25 @@ size_t tile_smem(int Lx, int Ly, int nfrag) {
                              2 * (size_t)most(y_doubles(Lx), y_doubles(Ly)));
 }
 
-void launch(const RealProblem& one, const RealProblem* d, int n, size_t smem, int grid, cudaStream_t st) {
+// the forms: one solve's chains over the grid, a cluster a chain, a cluster an image
+const auto grid_kernel = tile_sweep_kernel<kNT, 1, 352, true>;
+constexpr int kClusterMax = 128;                  // longest axis of the cluster forms
+const auto cluster_kernel = tile_sweep_kernel<kNT, 1, kClusterMax, false>;
+constexpr int kStringCtas = 4;                    // CTAs a chain, a cluster of 8 an image
+const auto string_kernel = tile_sweep_kernel<kStringNT, 3, kClusterMax, false>;
+
+cudaLaunchConfig_t cluster_config(int grid, int nt, int cluster, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3(kNT, 1, 1);
+    cfg.blockDim = dim3((unsigned)nt, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PS_CUDA(cudaLaunchKernelEx(&cfg, tile_sweep_kernel, one, d, n));
+    return cfg;
 }
 
 }  // namespace
@@ -632,30 +651,91 @@ size_t tile_sweep_smem(const RealProblem& p) { return tile_smem(p.Lx, p.Ly, p.nf
 
 int tile_sweep_tasks(int Lx, int Ly) { return std::max((Ly >= kLong ? kParts : 1) * ((Lx + 7) / 8), (Ly + 7) / 8); }
 
-bool tile_sweep_split(const RealProblem& p, int ncta) {
-    return p.Ly >= kLong && !p.os2 && ncta >= kParts * ((p.Lx + 7) / 8);
-}
-
 int tile_sweep_resident(size_t smem) {
     int dev = 0, sms = 0, occ = 0;
     PS_CUDA(cudaGetDevice(&dev));
     PS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PS_CUDA(cudaFuncSetAttribute(tile_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
-    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tile_sweep_kernel, kNT, smem));
+    PS_CUDA(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grid_kernel, kNT, smem));
     if (occ < 1) throw Error(-2, "sweep kernel does not fit on an SM");
     return sms * occ;
 }
 
 void tile_sweep_launch(const RealProblem& p0, int ncta, cudaStream_t st) {
     RealProblem p = p0;
-    p.cta0 = 0;
     p.ncta = ncta;
-    p.split = tile_sweep_split(p, ncta);
-    launch(p, nullptr, 0, tile_sweep_smem(p), ncta * p.nl, st);
+    // long rows in parts where that leaves no CTA two tasks: 128 x 352 13.4 us a step, whole 20.4
+    p.split = p.Ly >= kLong && !p.os2 && ncta >= kParts * ((p.Lx + 7) / 8);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ncta * p.nl), 1, 1);
+    cfg.blockDim = dim3(kNT, 1, 1);
+    cfg.dynamicSmemBytes = tile_sweep_smem(p);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PS_CUDA(cudaLaunchKernelEx(&cfg, grid_kernel, p, (const RealProblem*)nullptr));
 }
 
-void tile_sweep_launch_many(const RealProblem* d, int n, size_t smem, int grid, cudaStream_t st) {
-    launch(RealProblem{}, d, n, smem, grid, st);
+int tile_cluster_size(int Lx, int Ly) {
+    const int n = tile_sweep_tasks(Lx, Ly);
+    return Lx > kClusterMax || Ly > kClusterMax || n > 16 ? 0 : n > 8 ? 16 : 8;
+}
+
+int tile_cluster_resident(int cluster, size_t smem) {
+    PS_CUDA(cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+    PS_CUDA(cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(cluster, kNT, cluster, smem, nullptr, attr);
+    int n = 0;
+    PS_CUDA(cudaOccupancyMaxActiveClusters(&n, cluster_kernel, &cfg));
+    return n;
+}
+
+void tile_cluster_launch(const RealProblem& p, int cluster, cudaStream_t st) {
+    RealProblem one = p;
+    one.ncta = cluster;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(cluster * p.nl, kNT, cluster, tile_sweep_smem(p), st, attr);
+    PS_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel, one, (const RealProblem*)nullptr));
+}
+
+void tile_cluster_launch_many(const RealProblem* d, int n, int cluster, size_t smem, cudaStream_t st) {
+    RealProblem one{};
+    one.nl = 2;
+    one.ncta = cluster;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(n * 2 * cluster, kNT, cluster, smem, st, attr);
+    PS_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel, one, d));
+}
+
+bool tile_string_supported(int Lx, int Ly) {
+    return tile_sweep_supported(Lx, Ly) && Lx <= kClusterMax && Ly <= kClusterMax;
+}
+
+void tile_string_prepare(const RealProblem& p, int n) {
+    const size_t smem = tile_sweep_smem(p);
+    PS_CUDA(cudaFuncSetAttribute(string_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(n * 2 * kStringCtas, kStringNT, 2 * kStringCtas, smem, nullptr, attr);
+    int clusters = 0, per_sm = 0;
+    PS_CUDA(cudaOccupancyMaxActiveClusters(&clusters, string_kernel, &cfg));
+    PS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, string_kernel, kStringNT, smem));
+    char line[200];
+    std::snprintf(line, sizeof(line), "grid %dx%dx1 sweep in tiles: %d CTAs per problem, %d CTAs per SM, "
+                  "%d clusters resident at once, batch %d\n", p.Lx, p.Ly, 2 * kStringCtas, per_sm, clusters, n);
+    tuning_note(line);
+}
+
+void tile_string_launch(const RealProblem* d, int n, size_t smem, cudaStream_t st) {
+    RealProblem one{};
+    one.nl = 2;
+    one.ncta = kStringCtas;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(n * 2 * kStringCtas, kStringNT, 2 * kStringCtas, smem, st, attr);
+    PS_CUDA(cudaLaunchKernelEx(&cfg, string_kernel, one, d));
 }
 
 }  // namespace ps

@@ -43,8 +43,10 @@ def test_every_line_length_matches_oracle(ps, shape, scheme):
     assert np.abs(out - ref).max() < 1e-12 * np.abs(ref).max()
 
 
-def test_batch_members_equal_single_solves(ps):
+@pytest.mark.parametrize("extra", [0, 12])   # solves up to 64 x 64: with clusters for all of them, and with more
+def test_batch_members_equal_single_solves(ps, extra):
     shapes = [(64, 64, 1), (96, 128, 1), (128, 128, 1), (96, 16, 1), (128, 128, 1), (128, 64, 1), (48, 64, 1)]
+    shapes += extra * [(64, 64, 1)]
     specs = [dict(dim=2, shape=s, cell=ps.make_cell(2, "RECTANGULAR", 4.1, 3.6), Ms=(9 + 2 * (k % 3), 13), chiN=17.0)
              for k, s in enumerate(shapes)]
     rng = np.random.default_rng(5)
@@ -77,3 +79,19 @@ def test_adjoint_matches_line_passes(ps, shape, monkeypatch):
     # to the largest term, which exceeds the sum by less than 1e2: 1e2 x 64 x 50 eps < 1e-10
     for a, b in zip(*out):
         assert np.abs(a - b).max() < 1e-10 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("shape,mde", [((96, 64, 1), "RQM4"), ((12, 128, 1), "RQM4"), ((128, 96, 1), "OS2")])
+def test_string_images_equal_single_solves(ps, shape, mde):
+    n, cell = 5, ps.make_cell(2, "RECTANGULAR", 4.1, 3.6)
+    fields = 0.5 * np.random.default_rng(8).uniform(-1, 1, (2, n) + shape)
+    g = ps.StringAB(n, 2, shape, cell, (9, 13), 17.0, max_iter=2, mde=mde)
+    assert g.launches_per_iteration() < 30
+    g.set_images(*fields)
+    g.iterate(1)
+    phi = g.get("phiA")
+    for k in range(n):
+        m = ps.ModelAB(2, shape, cell, (9, 13), 17.0, mde=mde)
+        m.set_fields(fields[0, k], fields[1, k])
+        m.update(2)
+        assert np.array_equal(phi[k], m.get("phiA")), k
