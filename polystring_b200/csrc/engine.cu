@@ -222,6 +222,8 @@ PairChain::PairChain(int Lx, int Ly, int Lz, int scheme, int nbatch)
         if (nbatch != 1) throw Error(-2, "ETDRK4 chains are not batched");
         etd_.alloc(10 * (size_t)M_);
         for (int a = 0; a < plan_.naxes; a++) {
+            // a CTA an SM
+            set_tile_elems(plan_.ax[a], (int)std::min(2048L, std::max(256L, M_ / 148)));
             prepare_line_pass(MODE_FWD, plan_.ax[a]);
             prepare_line_pass(MODE_INV, plan_.ax[a]);
         }
@@ -266,8 +268,9 @@ void PairChain::set_tables_batched(const std::vector<double>& L1, const std::vec
 }
 
 int PairChain::launches_per_step() const {
-    // slices, 4 x (forward transform, combine, inverse transform), 3 nonlinear terms, store
-    if (scheme_ == SCHEME_ETDRK4) return 1 + 4 * (2 * plan_.naxes + 1) + 3 + 1;
+    // 1D: slices, 4 x (forward transform, combine, inverse transform), 3 nonlinear terms, store;
+    // else 4 x (spectral pass, passes along the middle axis, real pass)
+    if (scheme_ == SCHEME_ETDRK4) return plan_.naxes == 1 ? 17 : 4 * (2 * plan_.naxes - 2);
     if (plan_.naxes == 1) return 1;
     if (scheme_ == SCHEME_RQM4) return plan_.naxes == 3 ? 8 : 4;
     return plan_.naxes == 3 ? 4 : 2;

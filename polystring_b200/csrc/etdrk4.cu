@@ -13,13 +13,13 @@
 // with E = exp(ds L), E2 = exp(ds L / 2) and L = -k^2 (calc_k2_orthogonal).
 // Every spectral operation multiplies by real tables that are even in k, so
 // the packed field carries both lanes' spectra at once; the nonlinear term
-// takes each lane's own w.  Grids of up to 4096 points of 1D and 2D run all
-// steps in one CTA (etd_small_kernel); on others the transforms are the line
-// passes of line_pass.cu (MODE_FWD / MODE_INV over every axis) and the
-// elementwise work of the step is in the kernels below.
+// takes each lane's own w.  Grids of up to 1536 points of 1D and 2D run all
+// steps in one CTA (etd_small_kernel); on others a stage is two (2D) or four
+// (3D) passes (etd_pass_kernel).
 #include "engine.h"
 #include "fft_core.cuh"
 #include "ps_internal.h"
+#include "line_pass_body.cuh"
 
 #include <cmath>
 #include <complex>
@@ -73,31 +73,33 @@ __device__ __forceinline__ double2 lin2(double a, double2 x, double b, double2 y
 //   1: Na = T; T = E2 v + Q Na
 //   2: Nb = T; T = E2 a + Q (2 Nb - Nv)
 //   3: v = E v + f1 Nv + 2 f2 (Na + Nb) + f3 T; T = v
-__global__ void etd_combine_kernel(EtdFields f, long M, int stage) {
-    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < M; m += (long)gridDim.x * blockDim.x) {
-        const double2 t = f.T[m];
-        if (stage == 0) {
-            f.Nv[m] = t;
-            const double2 a = lin2(f.E2[m], f.V[m], f.Q[m], t);
-            f.A[m] = a;
-            f.T[m] = a;
-        } else if (stage == 1) {
-            f.Na[m] = t;
-            f.T[m] = lin2(f.E2[m], f.V[m], f.Q[m], t);
-        } else if (stage == 2) {
-            f.Nb[m] = t;
-            const double2 nv = f.Nv[m];
-            const double2 d = make_double2(2.0 * t.x - nv.x, 2.0 * t.y - nv.y);
-            f.T[m] = lin2(f.E2[m], f.A[m], f.Q[m], d);
-        } else {
-            const double2 v = f.V[m], nv = f.Nv[m], na = f.Na[m], nb = f.Nb[m];
-            const double e = f.E[m], g1 = f.f1[m], c2 = 2.0 * f.f2[m], g3 = f.f3[m];
-            const double2 r = make_double2(e * v.x + g1 * nv.x + c2 * (na.x + nb.x) + g3 * t.x,
-                                           e * v.y + g1 * nv.y + c2 * (na.y + nb.y) + g3 * t.y);
-            f.V[m] = r;
-            f.T[m] = r;
-        }
+__device__ __forceinline__ double2 etd_combine(const EtdFields& f, long m, int stage, double2 t) {
+    if (stage == 0) {
+        f.Nv[m] = t;
+        const double2 a = lin2(f.E2[m], f.V[m], f.Q[m], t);
+        f.A[m] = a;
+        return a;
     }
+    if (stage == 1) {
+        f.Na[m] = t;
+        return lin2(f.E2[m], f.V[m], f.Q[m], t);
+    }
+    if (stage == 2) {
+        f.Nb[m] = t;
+        const double2 nv = f.Nv[m];
+        const double2 d = make_double2(2.0 * t.x - nv.x, 2.0 * t.y - nv.y);
+        return lin2(f.E2[m], f.A[m], f.Q[m], d);
+    }
+    const double2 v = f.V[m], nv = f.Nv[m], na = f.Na[m], nb = f.Nb[m];
+    const double e = f.E[m], g1 = f.f1[m], c2 = 2.0 * f.f2[m], g3 = f.f3[m];
+    const double2 r = make_double2(e * v.x + g1 * nv.x + c2 * (na.x + nb.x) + g3 * t.x,
+                                   e * v.y + g1 * nv.y + c2 * (na.y + nb.y) + g3 * t.y);
+    f.V[m] = r;
+    return r;
+}
+__global__ void etd_combine_kernel(EtdFields f, long M, int stage) {
+    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < M; m += (long)gridDim.x * blockDim.x)
+        f.T[m] = etd_combine(f, m, stage, f.T[m]);
 }
 
 // q_f = Re(T) / M, q_c = Im(T) / M (q_c may be null)
@@ -111,24 +113,132 @@ __global__ void etd_store_kernel(const double2* __restrict__ T, double* __restri
 }
 
 // ---------------------------------------------------------------------------
+// 2D and 3D grids: a stage's two ends fused with the transforms along one axis
+// ---------------------------------------------------------------------------
+// The transforms' axes commute, so a stage's forward transform ends and its inverse
+// one begins along the last axis, and the inverse one ends and the next stage's
+// forward one begins along the first: with the spectral work between the former and
+// the nonlinear term between the latter, a stage is two launches (2D) or four (3D,
+// with the passes along the middle axis) where it was six or eight, and the field
+// makes as many round trips through L2.  Every launch and kernel of its own, a step
+// took 76 us at 128^2 (25 launches; now 31), 84 at 16^3 (33; 40), 101 at 32^3 (50),
+// 184 at 48^3 (93), 130 at 64^3 (85).  What bounds a launch is its latency (2.5 us at
+// 16^3, 5 at 64^3): tiles are small enough for a CTA an SM, and a launch starts before
+// the one ahead has ended (128^2 35 us a step without; letting it start as early as it
+// can costs 39, the waiting CTAs taking the running ones' places).
+struct EtdPass {
+    EtdFields f;
+    int stage;
+    const double *wf, *wc;   // w of the nonlinear term that follows (null: the sweep ends)
+    double *qf, *qc;         // the slices after the last stage
+    double M;
+};
+
+enum EtdKind {
+    ETD_SPEC,   // forward, spectral stage, inverse
+    ETD_REAL,   // inverse, nonlinear term (after the last stage: of the new slices), forward
+    ETD_FWD, ETD_INV
+};
+
+// A launch may start while the one before it ends: it reads the twiddles, then waits
+// for that launch's results.
+template <int N, int KIND>
+__global__ void __launch_bounds__(lp::kThreads) etd_pass_kernel(LineGeom g, EtdPass p, const double2* __restrict__ gtw) {
+    constexpr bool INV = KIND == ETD_REAL || KIND == ETD_INV;   // sign of the first transform
+    extern __shared__ __align__(16) double2 esm[];
+    double2 *twf = esm, *twi = esm + N, *A = esm + 2 * N, *B = A + N * g.LP;
+    for (int m = threadIdx.x; m < N; m += blockDim.x) {
+        const double2 t = gtw[m];
+        twf[m] = t;
+        twi[m] = make_double2(t.x, -t.y);
+    }
+    const lp::TileAddr ta = lp::tile_addr(g, blockIdx.x);
+    const int nel = N * g.T;
+    double2* const T = p.f.T;
+    using lp::kMaxEPT;
+    using lp::kThreads;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    PS_ELEMS(e) {
+        const lp::Elem el = lp::elem<N>(g, ta, e);
+        A[el.sidx] = T[el.goff];
+    }
+    __syncthreads();
+    double2* r = lp::tile_fft<N, INV ? +1 : -1>(A, B, g.T, g.LP, INV ? twi : twf);
+    if constexpr (KIND == ETD_SPEC || KIND == ETD_REAL) {
+        PS_ELEMS(e) {
+            const lp::Elem el = lp::elem<N>(g, ta, e);
+            if constexpr (KIND == ETD_REAL) {
+                const double xf = r[el.sidx].x / p.M, xc = r[el.sidx].y / p.M;
+                if (p.stage == 3) {
+                    p.qf[el.goff] = xf;
+                    p.qc[el.goff] = xc;
+                }
+                if (p.wf) r[el.sidx] = make_double2(-p.wf[el.goff] * xf, -p.wc[el.goff] * xc);
+            } else {
+                r[el.sidx] = etd_combine(p.f, el.goff, p.stage, r[el.sidx]);
+            }
+        }
+        if (KIND == ETD_REAL && !p.wf) return;
+        __syncthreads();
+        r = lp::tile_fft<N, INV ? -1 : +1>(r, lp::other(r, A, B), g.T, g.LP, INV ? twf : twi);
+    }
+    asm volatile("griddepcontrol.launch_dependents;");
+    PS_ELEMS(e) {
+        const lp::Elem el = lp::elem<N>(g, ta, e);
+        T[el.goff] = r[el.sidx];
+    }
+}
+
+size_t etd_pass_smem(const LineGeom& g) { return sizeof(double2) * (2 * (size_t)g.N + 2 * (size_t)g.N * g.LP); }
+
+template <int N, int KIND>
+void etd_pass_n(const LineGeom& g, const EtdPass* p, cudaStream_t st) {
+    const auto k = etd_pass_kernel<N, KIND>;
+    if (!p) {
+        PS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLinePassSmemLimit));
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g.ntiles, 1, 1);
+    cfg.blockDim = dim3(lp::kThreads, 1, 1);
+    cfg.dynamicSmemBytes = etd_pass_smem(g);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PS_CUDA(cudaLaunchKernelEx(&cfg, k, g, *p, twiddle_table(N)));
+}
+
+// launches the pass, or (p == nullptr) sets its kernel's attributes
+template <int KIND>
+void etd_pass(const LineGeom& g, const EtdPass* p, cudaStream_t st) {
+    switch (g.N) {
+#define X(N) case N: return etd_pass_n<N, KIND>(g, p, st);
+        X(2) X(4) X(8) X(12) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(352)
+#undef X
+    }
+}
+
+// ---------------------------------------------------------------------------
 // small grids: all steps in one CTA
 // ---------------------------------------------------------------------------
 // The packed field ping-pongs between two shared-memory buffers, one Stockham
 // radix pass a barrier; element (x, y) sits at x P + y with an odd pitch P, so
 // that threads on consecutive lines of either axis fall in different banks.
-// The spectral fields of a point belong to one thread for the whole solve: in
-// registers up to 4 points a thread, else in the chain's scratch fields.
+// The spectral fields of a point stay in the registers of its thread for the whole
+// solve.
 // What bounds it is the chain of 8 transforms a step, each radix pass some 400
 // cycles of shared-memory and FP64 latency and a barrier: 32^2 16.7 us a step,
-// 1D 64 points 5.0 us (by line passes 33 and 17 launches, 59 and 33 us).
-constexpr long kSmallPoints = 4096;
+// 1D 64 points 5.0 us (by passes 26 and 33).
+constexpr long kSmallPoints = 1536;   // 32 x 48 27.0 us a step, by passes 27.9; 32 x 64 31.5 and 27.8
 
 struct EtdSmall {
     double *hf, *hc;              // histories; hc == nullptr: lane c carries nothing
     const double *wf[2], *wc[2];  // w of each lane before and from its switch step
     int swf, swc, nsteps, Lx, Ly;
     const double *E, *E2, *Q, *f1, *f2, *f3;
-    double2 *V, *Nv, *A, *S;      // scratch fields (more than 4 points a thread)
     const double2 *twx, *twy;
 };
 
@@ -190,7 +300,7 @@ template <int NT, int KP>
 __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant__ EtdSmall a) {
     // the spectral fields in registers, and with the registers of up to 256
     // threads the tables and w as well (read from the L2 twice a stage otherwise)
-    constexpr bool REGS = KP <= 4, TAB = REGS && NT <= 256;
+    constexpr bool TAB = NT <= 256;
     const int M = a.Lx * a.Ly, P = a.Ly | 1, F = a.Lx * P;
     auto magic = [](int n) { return (unsigned)(((1ull << 32) + n - 1) / n); };
     const SmallAxis ax = {a.Lx, a.Ly, 1, P, 0, magic(a.Ly)}, ay = {a.Ly, a.Lx, P, 1, a.Lx, magic(a.Lx)};
@@ -200,7 +310,7 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
         for (int i = threadIdx.x; i < a.Ly; i += NT) esm[a.Lx + i] = a.twy[i];
     const double Md = (double)M, rM = 1.0 / Md;
     const bool pow2 = (M & (M - 1)) == 0;
-    double2 rV[REGS ? KP : 1], rN[REGS ? KP : 1], rA[REGS ? KP : 1], rS[REGS ? KP : 1];
+    double2 rV[KP], rN[KP], rA[KP], rS[KP];
     int place[KP];
 #pragma unroll
     for (int k = 0; k < KP; k++) {
@@ -214,10 +324,6 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
             if (m < M) f(k, m, place[k]);
         }
     };
-    auto V = [&](int k, int m) -> double2& { if constexpr (REGS) return rV[k]; else return a.V[m]; };
-    auto Nv = [&](int k, int m) -> double2& { if constexpr (REGS) return rN[k]; else return a.Nv[m]; };
-    auto A = [&](int k, int m) -> double2& { if constexpr (REGS) return rA[k]; else return a.A[m]; };
-    auto S = [&](int k, int m) -> double2& { if constexpr (REGS) return rS[k]; else return a.S[m]; };
     auto flip = [&](bool moved) {
         if (moved) {
             const int c = cur;
@@ -235,7 +341,7 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
         flip(small_axis<+1, NT>(cur, oth, ax));
         if (a.Ly > 1) flip(small_axis<+1, NT>(cur, oth, ay));
     };
-    double2 q[REGS ? KP : 1];   // the slice (more points: read back from the history)
+    double2 q[KP];   // the slice
     double tab[6][TAB ? KP : 1], w[2][TAB ? KP : 1];
     const double* const tabs[6] = {a.E, a.E2, a.Q, a.f1, a.f2, a.f3};
     if constexpr (TAB)
@@ -255,12 +361,12 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
         if (t == 0 || t == a.swf || t == a.swc) {
             each([&](int, int m, int i) { esm[cur + i] = make_double2(qf[m], qc ? qc[m] : 0.0); });
             forward();
-            each([&](int k, int m, int i) { V(k, m) = esm[cur + i]; });
+            each([&](int k, int, int i) { rV[k] = esm[cur + i]; });
         }
         each([&](int k, int m, int i) {
             double2 x;
-            if (!REGS || t == 0) x = make_double2(qf[m], qc ? qc[m] : 0.0);
-            else x = q[REGS ? k : 0];
+            if (t == 0) x = make_double2(qf[m], qc ? qc[m] : 0.0);
+            else x = q[k];
             esm[cur + i] = make_double2(-W(0, k, m) * x.x, qc ? -W(1, k, m) * x.y : 0.0);
         });
 #pragma unroll 1
@@ -276,21 +382,21 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
                 const double2 z = esm[cur + i];
                 double2 r;
                 if (stage == 0) {
-                    Nv(k, m) = z;
-                    r = lin2(T(1, k, m), V(k, m), T(2, k, m), z);
-                    A(k, m) = r;
+                    rN[k] = z;
+                    r = lin2(T(1, k, m), rV[k], T(2, k, m), z);
+                    rA[k] = r;
                 } else if (stage == 1) {
-                    S(k, m) = z;
-                    r = lin2(T(1, k, m), V(k, m), T(2, k, m), z);
+                    rS[k] = z;
+                    r = lin2(T(1, k, m), rV[k], T(2, k, m), z);
                 } else if (stage == 2) {
-                    const double2 nv = Nv(k, m), na = S(k, m);
-                    S(k, m) = make_double2(na.x + z.x, na.y + z.y);
-                    r = lin2(T(1, k, m), A(k, m), T(2, k, m), make_double2(2.0 * z.x - nv.x, 2.0 * z.y - nv.y));
+                    const double2 nv = rN[k], na = rS[k];
+                    rS[k] = make_double2(na.x + z.x, na.y + z.y);
+                    r = lin2(T(1, k, m), rA[k], T(2, k, m), make_double2(2.0 * z.x - nv.x, 2.0 * z.y - nv.y));
                 } else {
-                    const double2 v = V(k, m), nv = Nv(k, m), s = S(k, m);
+                    const double2 v = rV[k], nv = rN[k], s = rS[k];
                     const double e = T(0, k, m), g1 = T(3, k, m), c2 = 2.0 * T(4, k, m), g3 = T(5, k, m);
                     r = make_double2(e * v.x + g1 * nv.x + c2 * s.x + g3 * z.x, e * v.y + g1 * nv.y + c2 * s.y + g3 * z.y);
-                    V(k, m) = r;
+                    rV[k] = r;
                 }
                 esm[cur + i] = r;
             });
@@ -302,7 +408,7 @@ __global__ void __launch_bounds__(NT, 1) etd_small_kernel(const __grid_constant_
             const double2 x = make_double2(div_pow2_or_rn(z.x, Md, rM, pow2), div_pow2_or_rn(z.y, Md, rM, pow2));
             of[m] = x.x;
             if (oc) oc[m] = x.y;
-            if constexpr (REGS) q[k] = x;
+            q[k] = x;
         });
     }
 }
@@ -318,8 +424,7 @@ template <class F>
 void small_kernel(long M, F f) {
     if (M <= 128) f(etd_small_kernel<64, 2>, 64);
     else if (M <= 1024) f(etd_small_kernel<256, 4>, 256);
-    else if (M <= 2048) f(etd_small_kernel<512, 4>, 512);
-    else f(etd_small_kernel<512, 8>, 512);
+    else f(etd_small_kernel<512, 3>, 512);
 }
 
 }  // namespace
@@ -361,6 +466,12 @@ void PairChain::set_tables_etd(const std::vector<double>& k2, double ds, int Mc)
         small_kernel(M_, [](auto kernel, int) {
             PS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         });
+    }
+    for (int a = 0; a < plan_.naxes; a++) {
+        etd_pass<ETD_SPEC>(plan_.ax[a], nullptr, nullptr);
+        etd_pass<ETD_REAL>(plan_.ax[a], nullptr, nullptr);
+        etd_pass<ETD_FWD>(plan_.ax[a], nullptr, nullptr);
+        etd_pass<ETD_INV>(plan_.ax[a], nullptr, nullptr);
     }
     etdtab_.alloc(tab.size());
     PS_CUDA(cudaMemcpy(etdtab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
@@ -408,13 +519,45 @@ void PairChain::enqueue_etd(double* hf, double* hc, int nsteps, const LaneFactor
         a.swf = lf.switch_t; a.swc = lc.switch_t;
         a.nsteps = nsteps; a.Lx = Lx_; a.Ly = Ly_;
         a.E = f.E; a.E2 = f.E2; a.Q = f.Q; a.f1 = f.f1; a.f2 = f.f2; a.f3 = f.f3;
-        a.V = f.V; a.Nv = f.Nv; a.A = f.A; a.S = f.Na;
         a.twx = twiddle_table(Lx_);
         a.twy = Ly_ > 1 ? twiddle_table(Ly_) : nullptr;
         small_kernel(M, [&](auto kernel, int threads) {
             kernel<<<1, threads, small_smem(Lx_, Ly_), st>>>(a);
         });
         PS_CUDA(cudaGetLastError());
+        return;
+    }
+    if (plan_.naxes > 1) {
+        const LineGeom &in = plan_.ax[0], &out = plan_.ax[plan_.naxes - 1];
+        EtdPass p{};
+        p.f = f;
+        p.M = rM;
+        for (int t = 0; t < nsteps; t++) {
+            const double* qf = hf + (long)t * M;
+            const double* qc = c_in_fixed ? c_in_fixed : hc + (long)t * M;
+            if (t == 0 || t == lf.switch_t || t == lc.switch_t) {
+                etd_slices_kernel<<<nb, kEtdThreads, 0, st>>>(f.V, qf, qc, nullptr, nullptr, M, 0);
+                PS_CUDA(cudaGetLastError());
+                transform(f.V, MODE_FWD, st);
+            }
+            if (t == 0) {
+                etd_slices_kernel<<<nb, kEtdThreads, 0, st>>>(T, qf, qc, lf.F(0), lc.F(0), M, 1);
+                PS_CUDA(cudaGetLastError());
+                etd_pass<ETD_FWD>(in, &p, st);
+            }
+            for (int stage = 0; stage < 4; stage++) {
+                const bool last = stage == 3, next = !last || t + 1 < nsteps;
+                p.stage = stage;
+                p.wf = next ? lf.F(last ? t + 1 : t) : nullptr;
+                p.wc = next ? lc.F(last ? t + 1 : t) : nullptr;
+                p.qf = hf + (long)(t + 1) * M;
+                p.qc = c_in_fixed ? c_out_fixed : hc + (long)(t + 1) * M;
+                if (plan_.naxes > 2) etd_pass<ETD_FWD>(plan_.ax[1], &p, st);
+                etd_pass<ETD_SPEC>(out, &p, st);
+                if (plan_.naxes > 2) etd_pass<ETD_INV>(plan_.ax[1], &p, st);
+                etd_pass<ETD_REAL>(in, &p, st);
+            }
+        }
         return;
     }
     for (int t = 0; t < nsteps; t++) {

@@ -1,4 +1,4 @@
-"""ETDRK4 solves that run in one CTA (1D and 2D grids up to 4096 points) at the
+"""ETDRK4 solves that run in one CTA (1D and 2D grids up to 1536 points) at the
 edges of their kernels' ranges, both chains, against the line passes: the same
 operations on the same values, other radix schedules."""
 import numpy as np
@@ -14,7 +14,7 @@ def ps():
 
 
 @pytest.mark.parametrize("shape", [(2, 1, 1), (64, 1, 1), (128, 1, 1), (352, 1, 1), (2, 2, 1), (12, 24, 1), (32, 32, 1),
-                                   (48, 24, 1), (128, 16, 1), (64, 48, 1), (64, 64, 1)])
+                                   (48, 24, 1), (128, 12, 1), (32, 48, 1)])
 def test_small_grids_match_line_passes(ps, monkeypatch, shape):
     dim = 1 if shape[1] == 1 else 2
     rng = np.random.default_rng(4)
