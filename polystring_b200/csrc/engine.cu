@@ -480,7 +480,7 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     }
     PS_CUDA(cudaStreamSynchronize(st_));
     launches_per_prop_ = real_ || chain_->small_etd() ? 1 : chain_->launches_per_step() * Ns_ + (chain_->plan().naxes > 1 ? 1 : 0);
-    launches_per_iter_ = launches_per_prop_ + 2 + 2 + (p.scft == 1 ? 4 : 1);
+    launches_per_iter_ = launches_per_prop_ + mean_launches(M_) + density_launches(M_, 2) + (p.scft == 1 ? 4 : 1);
 }
 
 ModelAB::~ModelAB() {
@@ -560,8 +560,9 @@ void ModelAB::enqueue_densities(cudaStream_t st) {
     double* dQ = scal_.p + 0;
     launch_mean(hf_.p + (long)Ns_ * M_, M_, partial_.p, dQ, st);
     // phiA = (1/Q) dsA sum c_s qA[s] qAc[LA - s]; phiB likewise (Model_AB.cc:196-199)
-    launch_density(hf_.p, hc_.p + (long)LB_ * M_, LA_, M_, cA_.p, dsA_, dQ, 0.0, phiA_.p, 1, 0, 0, nullptr, st);
-    launch_density(hf_.p + (long)LA_ * M_, hc_.p, LB_, M_, cB_.p, dsB_, dQ, 0.0, phiB_.p, 1, 0, 0, nullptr, st);
+    const DensityJobs jobs{{{hf_.p, hc_.p + (long)LB_ * M_, cA_.p, LA_, dsA_, phiA_.p},
+                            {hf_.p + (long)LA_ * M_, hc_.p, cB_.p, LB_, dsB_, phiB_.p}}};
+    launch_densities(jobs, 2, M_, dQ, st);
 }
 
 void ModelAB::enqueue_post(cudaStream_t st) {

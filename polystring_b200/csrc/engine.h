@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "ps_internal.h"
+#include "field_kernels.h"
 #include "anderson.h"
 #include "real_sweep.h"
 
@@ -300,7 +301,7 @@ public:
     const double* factor(int full, int block) const { return full ? eF_[block].p : eH_[block].p; }
     void enqueue_propagate(cudaStream_t s);
     void enqueue_post(cudaStream_t s);
-    int launches_post() const { return 2 + 3 + (p_.scft == 1 ? 4 : 1); }
+    int launches_post() const { return mean_launches(M_) + density_launches(M_, 3) + (p_.scft == 1 ? 4 : 1); }
     // the persistent sweep with three factor sets
     bool persistent_sweep() const { return real_ != nullptr; }
     const RealSweep* sweep() const { return real_; }

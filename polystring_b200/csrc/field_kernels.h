@@ -7,6 +7,8 @@ namespace ps {
 
 constexpr int kRedBlocks = 296;   // 2 x 148 SMs
 constexpr int kRedThreads = 256;
+constexpr long kOneBlockPoints = 4096;   // reductions of up to that many points: one launch
+inline int mean_launches(long M) { return M <= kOneBlockPoints ? 1 : 2; }
 constexpr int kRedMaxK = 11;      // widest fixed reduction (triblock EM residual)
 
 struct EMArgs {
@@ -50,6 +52,19 @@ void launch_residual_ax_abc(const double* const d[3], const double* const w[3], 
                             double* out6, cudaStream_t st);
 void launch_em_update_abc(const EMABCArgs& a, cudaStream_t st);
 void launch_arc_sq(const double* a, const double* b, long M, double* partial, double* out, cudaStream_t st);
+// one block's density: phi = cc ds sum_s c[s] q[s] qc[n - s]
+struct DensityJob {
+    const double *q, *qc, *c;
+    int n;
+    double ds;
+    double* phi;
+};
+struct DensityJobs { DensityJob job[3]; };
+// the densities of a solve's blocks, cc = 1 / *Qdev: in one launch on small grids
+// (an iteration after its sweep: 96^2 14.5 us in one, 16.6 in two; 32^3 18.6 in both;
+// 48^3 44.2 and 41.1)
+inline int density_launches(long M, int njobs) { return M < 32 * 32 * 32 ? 1 : njobs; }
+void launch_densities(const DensityJobs& jobs, int njobs, long M, const double* Qdev, cudaStream_t st);
 void launch_density(const double* q, const double* qc, int n, long M, const double* c, double ds,
                     const double* Qdev, double cc_host, double* phi, int nbatch, long bstride_q, long bstride_phi,
                     const double* Qbatch, cudaStream_t st);

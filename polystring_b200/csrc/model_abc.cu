@@ -21,10 +21,9 @@
 //     coefficient set from U = UA + UB + UC, V = VA + VB + VC;
 //   * Hw = mean(chiAB phiA phiB + chiBC phiB phiC + chiAC phiA phiC -
 //     sum_X wX phiX), Hs = -ln Q; the residuals of Model_AB with a third field.
-// Incompressible, RQM4, orthogonal k^2 table.  Propagation: the 64^3 sweep
-// (sweep64.cu) on 64^3 grids and the generic persistent sweep (sweep.cu) on
-// 32^3 and 48^3 grids, each given three factor sets; the packed line passes
-// (PairChain) on other grids.
+// Incompressible, RQM4, orthogonal k^2 table.  Propagation: the persistent sweeps
+// (RealSweep) given three factor sets, the packed line passes (PairChain) on grids
+// that have none.
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -158,11 +157,12 @@ void ModelABC::enqueue_post(cudaStream_t st) {
     // block X spans forward slices [oX, oX + LX]; its complementary slices
     // run backwards from Ns - oX
     const long o[3] = {0, L_[0], (long)L_[0] + L_[1]};
+    DensityJobs jobs;
     for (int x = 0; x < 3; x++) {
         const long oc = Ns_ - o[x] - L_[x];
-        launch_density(hf_.p + o[x] * M_, hc_.p + oc * M_, L_[x], M_, c_[x].p, ds_[x], dQ, 0.0, phi_[x].p, 1, 0, 0,
-                       nullptr, st);
+        jobs.job[x] = {hf_.p + o[x] * M_, hc_.p + oc * M_, c_[x].p, L_[x], ds_[x], phi_[x].p};
     }
+    launch_densities(jobs, 3, M_, dQ, st);
     if (p_.scft == 1) {
         AXArgs a{};
         a.state = axs_; a.n = p_.n_anderson; a.M = M_; a.nf = 3;
