@@ -76,9 +76,9 @@ def fp64_peak_tflops(ps):
 
 
 def traffic_per_gridpt_step():
-    """DRAM bytes per gridpoint-step of the propagator line passes from the
+    """DRAM bytes per gridpoint-step of the propagator sweep from the
     committed ncu summary (None until one exists)."""
-    path = os.path.join(ROOT, "profiles", "propagator_sweep64_c2_64cube.txt")
+    path = os.path.join(ROOT, "profiles", "real_sweep_64cube.txt")
     try:
         with open(path) as f:
             for line in f:

@@ -15,12 +15,15 @@
 //
 // OS2 has only the W warps' operators, with q = e^{-w ds/2} Dy(full) W.
 // One SM's tensor cores bound a 64^2 step at 6 operators x 8 tiles x 670 cycles
-// / 4 = 8000 cycles (4.2 us).
+// / 4 = 8000 cycles (4.2 us); it takes 9.1, 48^2 5.4, 32^2 2.3, 16^2 1.2 (a launch
+// per line pass: 64^2 20).  So single solves leave it for the tiles of tile_sweep.cu
+// from 32 x 64 points on, while batches and strings, whose chains fill the SMs, stay.
 //
 // 1D: thread (chain, orbit) keeps the orbit's four points of q and the factors
 // in registers; an operator's folded values go through shared memory, its
 // (block, output tile) products belong to one warp each, the two chains being
-// two of the eight lines of a product.
+// two of the eight lines of a product.  64 points 0.84 us a step (a launch a step: 10),
+// 128 1.6, 256 5.6; its chain of shared-memory trips bounds it.
 #include <algorithm>
 
 #include "engine.h"

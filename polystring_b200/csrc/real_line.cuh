@@ -128,38 +128,6 @@ struct RealLine {
         }
         unfold(x);
     }
-
-    // The same with the blocks formed from their Toeplitz and Hankel parts (see
-    // real_parts): one load and one addition a fragment instead of one load, and
-    // 2 KB of tables an operator at N = 128 instead of 32 KB of fragments.  th is
-    // the operator's table; lanes read consecutive doubles around one entry.
-    __device__ __forceinline__ static void apply_parts(double (&x)[E], const double* th) {
-        const int lane = threadIdx.x & 31, og = real_column_orbit(lane >> 2), j = lane & 3;
-        if constexpr (!WHOLE) {
-            // the parts go on past the last orbit: what the lane holds there counts as zero
-#pragma unroll
-            for (int b = 0; b < 4; b++) x[4 * (S - 1) + b] = j + 4 * (S - 1) < O ? x[4 * (S - 1) + b] : 0.0;
-        }
-        fold(x);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const double* tp = th + 2 * h * PARTS + 4 * S + og - j;
-            const double* hp = th + (2 * h + 1) * PARTS + og + j + 1;
-            double y[4 * T];
-#pragma unroll
-            for (int i = 0; i < 4 * T; i++) y[i] = 0.0;
-#pragma unroll
-            for (int s = 0; s < S; s++)
-#pragma unroll
-                for (int t = 0; t < T; t++) {
-                    const double a = tp[8 * t - 4 * s], b = hp[8 * t + 4 * s];
-                    mma(y[2 * t], y[2 * t + 1], x[4 * s + 2 * h], a + b);
-                    mma(y[2 * T + 2 * t], y[2 * T + 2 * t + 1], x[4 * s + 2 * h + 1], a - b);
-                }
-            join(y, h, x);
-        }
-        unfold(x);
-    }
 #endif
 };
 
@@ -209,7 +177,9 @@ inline void real_fragments(int N, const std::vector<double>& L, std::vector<doub
 PS_HD constexpr int real_parts_doubles(int N) { return 4 * (8 * ((N / 4 + 7) / 8) + 4 * ((N / 4 + 3) / 4)); }
 
 // appends the parts of the same operator's blocks: for s = +1, -1 the Toeplitz
-// part T_s(d) / 4 at 4 S + d, then the Hankel part T_s(d) / 4 at d
+// part T_s(d) / 4 at 4 S + d, then the Hankel part T_s(d) / 4 at d.  A fragment is
+// their sum (r = +1) or difference: an addition more than reading it, but 2 KB an
+// operator at 128 points instead of 32 KB.
 inline void real_parts(int N, const std::vector<double>& L, std::vector<double>& out) {
     const int O = N / 4, S = (O + 3) / 4, T = (O + 7) / 8, n = 8 * T + 4 * S;
     const RealKernel Ts(N, L);

@@ -21,6 +21,17 @@
 // one warp, whose arithmetic does not depend on how tasks are spread over warps
 // and CTAs: a solve in a shared launch equals its single launch bit for bit.
 //
+// us a contour step, RQM4 both chains: 16^3 5.7, 32^3 7.3 (38 with packed complex
+// FFTs in four phases), 48^3 12.3 (57), 64^3 17.5 (21.2 in clusters of two CTAs), 48 x
+// 64 x 32 10.4 (one chain in a launch per line pass: 29).  What bounds it: small grids the two
+// barriers (1.4 us and the slowest CTA each) and the phases' chains of L2 reads,
+// products and writes; 64^3 the L2, which the x-pass reads and writes at 6 TB/s
+// (7300 cycles of which 5300 remain without arithmetic), and the products of the
+// plane, 40 % of the FP64 tensor peak while they run.  One CTA of 256 threads an SM:
+// with 255 registers each the next operands are prefetched; 512 threads spill, two
+// CTAs an SM gain nothing alone (19 to 20 us at 64^3), a barrier a field costs 10.2 us
+// at 32^3, two columns a lane 19.1 at 64^3.
+//
 // Barriers count arrivals per solve with a bounded spin; the launch is
 // cooperative, so all CTAs are resident.  On a timeout the CTA raises the error
 // flag, every CTA of the solve sees it and returns, and the host reports it.

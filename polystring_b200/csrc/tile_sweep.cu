@@ -13,14 +13,25 @@
 //             Z = Dy(half) e^{-w ds/4} q
 //
 // OS2 has only W.  Thread (line, orbit) holds an orbit's four points in
-// registers; folded values go through shared memory to the warps, warp k
-// computing the products k, k + 8, ... of (character pair, output tile), and the
+// registers; folded values go through shared memory to the warps, which share the
+// products of (field, character s, J output tiles) so that each has one unit, and the
 // results back.  So a line of 128 points takes eight warps some 300 cycles where
 // one warp alone takes 2800, which is what a single solve's few lines need.
 // Lines of up to 64 points read the blocks' fragments (16 KB an operator pair at
 // 64), longer ones form them from the Toeplitz and Hankel parts (4 KB at 128 points
-// where the fragments take 64 KB).  The arithmetic of a line does not depend on how tiles
-// are spread over CTAs.
+// where the fragments take 64 KB).  The arithmetic of a line does not depend on how
+// tiles are spread over CTAs or threads, and is that of plane_sweep.cu.
+//
+// Three forms.  A chain of up to 16 tiles is a cluster with the hardware's barrier
+// (us a step: 64^2 4.4, 96^2 6.4, 128^2 6.8; with the barrier in memory, 1.4 us each,
+// 5.9, 7.2, 8.3; line passes 20, 21.3, 22.4; 128^2 with 8 CTAs 11.9, so it takes 16).
+// Larger grids run over the whole grid with barriers in memory, rows of 256 points on
+// in parts (128 x 352 13.4, whole 20.4, line passes 26.5; 256^2 18.2, 28.5).  An image
+// of a string is a cluster of eight CTAs of 128 threads, three an SM, so that 40
+// images are resident at once (96^2 28.9 us a step for all, line passes 48.5; 16 x 128
+// 12.4 and 26).  What bounds the first two is latency: two barriers and four trips
+// through L2 and shared memory a step beside 1.6 us of products (128^2); strings the
+// L2, some 3 TB/s of field traffic, and the trips.
 #include <algorithm>
 #include <cstdio>
 

@@ -237,7 +237,7 @@ def run_once(name):
     device: 'sweep64' (the C2 64^3 model with Ms [21, 41], 244 MB of
     histories, three iterations: one 64^3 sweep launch each) and 'string12'
     (12 images of 128^2, Ns 128, three string iterations of one SCFT
-    iteration each: one cluster-sweep launch each)."""
+    iteration each: one sweep launch each)."""
     import polystring_b200 as ps
     if name == "sweep64":
         c = config("C2")

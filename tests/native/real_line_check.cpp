@@ -23,7 +23,7 @@ double check() {
     std::vector<double> th;
     real_parts(N, L, th);
     if ((int)th.size() != 4 * R::PARTS || (int)th.size() != real_parts_doubles(N)) return 3.0;
-    double parts = 0.0;   // fragments formed from the parts, as apply_parts() reads them
+    double parts = 0.0;   // fragments formed from the parts, sums and differences of table entries
     for (int b = 0; b < 4; b++)
         for (int t = 0; t < R::T; t++)
             for (int s = 0; s < R::S; s++)
