@@ -68,18 +68,39 @@ __global__ void __launch_bounds__(kRedThreads) reduce_final_kernel(const double*
 
 // Small fields in one launch of one block, whose reads cost less than a second launch:
 // with the densities in one launch too, an iteration after its sweep (simple mixing)
-// takes 10.3 us at 64 points of 1D, 12.4 at 64^2 and 16^3; in two and two 12.4 and 16.5.
+// takes 10.3 us at 64 points of 1D and 12.4 to 13.4 at 32^2, in two and two 12.4 and
+// 16.5.  At 4096 points a block's four rounds of reads cost the launch: 16.5, in two 14.5.
+// The order of the sums is that of the two launches, whose blocks then have at most
+// one point a thread.
 template <class F, int K>
 __global__ void __launch_bounds__(kRedThreads) reduce_one_kernel(F f, long M, double scale, double* out) {
+    constexpr int B = (int)(kOneBlockPoints / kRedThreads), W = kRedThreads / 32;
+    static_assert(B <= kRedBlocks && B <= kRedThreads, "a block of the first launch a chunk");
+    __shared__ double sh[B][K][W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 4
+    for (int b = 0; b < B; b++) {
+        const long i = (long)b * kRedThreads + threadIdx.x;
+        if ((long)b * kRedThreads >= M) break;
+        double v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = 0.0;
+        if (i < M) f(i, v);
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            double s = 0.0 + v[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0) sh[b][k][warp] = s;
+        }
+    }
+    __syncthreads();
     double acc[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) acc[k] = 0.0;
-#pragma unroll 4
-    for (long i = threadIdx.x; i < M; i += kRedThreads) {
-        double v[K];
-        f(i, v);
-#pragma unroll
-        for (int k = 0; k < K; k++) acc[k] += v[k];
+    for (int k = 0; k < K; k++) {
+        acc[k] = 0.0;
+        if ((long)threadIdx.x * kRedThreads < M && threadIdx.x < B)
+            for (int w = 0; w < W; w++) acc[k] += sh[threadIdx.x][k][w];
     }
     __shared__ double res[K];
     block_reduce_store<K>(acc, res);

@@ -7,7 +7,7 @@ namespace ps {
 
 constexpr int kRedBlocks = 296;   // 2 x 148 SMs
 constexpr int kRedThreads = 256;
-constexpr long kOneBlockPoints = 4096;   // reductions of up to that many points: one launch
+constexpr long kOneBlockPoints = 1024;   // reductions of up to that many points: one launch
 inline int mean_launches(long M) { return M <= kOneBlockPoints ? 1 : 2; }
 constexpr int kRedMaxK = 11;      // widest fixed reduction (triblock EM residual)
 

@@ -1,5 +1,5 @@
 """Q and the densities on both sides of the sizes where their launches change (fields
-of up to 4096 points reduced by one block, densities of grids below 32768 points in
+of up to 1024 points reduced by one block, densities of grids below 32768 points in
 one launch) against the contour sums of the returned propagators."""
 import numpy as np
 import pytest
@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(4, 1, 1), (256, 1, 1), (64, 64, 1), (48, 96, 1), (16, 16, 16), (16, 16, 24),
+@pytest.mark.parametrize("shape", [(4, 1, 1), (256, 1, 1), (32, 32, 1), (48, 24, 1), (16, 16, 4), (16, 16, 24),
                                    (32, 32, 24), (32, 32, 32)])
 @pytest.mark.parametrize("blocks", [2, 3])
 def test_Q_and_densities(shape, blocks):
