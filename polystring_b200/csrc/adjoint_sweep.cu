@@ -228,9 +228,11 @@ void stress_launch(const StressArgs& a, cudaStream_t st) {
 
 // The chains' kept fields (and with `grad` the adjoint chains) of all steps:
 // 4 (10) Ns M doubles beside the 2 (Ns + 1) M of the histories.  False where
-// the grid has no sweep or the device has no room: the line passes serve then.
+// the grid has no sweep that keeps them (one with a single axis longer than a point,
+// in a cell of any dimension, has not) or the device has no room: the line passes
+// serve then, or refuse the grid.
 bool ModelAB::sweep_adjoint(bool grad) {
-    if (!real_ || p_.dim < 2) return false;
+    if (!real_ || chain_->plan().naxes < 2) return false;
     // the stress keeps an axis's operator in shared memory: 36 KB at 128 points, 250 KB at 352
     if (!grad && (p_.Lx > 128 || p_.Ly > 128 || p_.Lz > 128)) return false;
     const size_t n = (size_t)Ns_ * M_;

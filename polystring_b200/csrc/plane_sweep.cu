@@ -443,6 +443,8 @@ bool line_sweep_supported(int Lx) {
 }
 
 void line_sweep_launch(const RealProblem& p, cudaStream_t st) {
+    for (const RealLane& L : p.lane)
+        if (L.keep_half || L.keep_full || L.src_o) throw Error(-2, "the sweep of 1D grids keeps no fields and takes no source");
     switch (p.Lx) {
 #define X(V) case V: line_sweep_kernel<V><<<1, k1T, 0, st>>>(p); break;
         LN_CASES(X)
