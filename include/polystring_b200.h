@@ -20,6 +20,12 @@
  * and return without synchronising; the others take host pointers and
  * return after the result is in host memory.
  *
+ * A sweep over many CTAs that are kept from running together (by another program's
+ * kernels, say) gives up at its grid barrier after some ten seconds
+ * (PS_B200_BARRIER_POLLS=n: after n polls).  The model's and batch's calls that wait
+ * for results, and the next iteration, then return PS_ERR_CUDA until fields are set
+ * again; an updater's see ps_updater_check.
+ *
  * Paths in the citations are relative to the reference project root.
  */
 #ifndef POLYSTRING_B200_H
@@ -122,6 +128,11 @@ void ps_updater_destroy(ps_updater* u);
  * entry; slices 1..len-1 are overwritten. */
 int ps_updater_solve(ps_updater* u, const double* w, double* qs, int len);
 int ps_updater_solve_device(ps_updater* u, const double* w, double* qs, int len, void* stream);
+/* No counterpart in the reference.  PS_OK, or PS_ERR_CUDA (once) if a solve of this
+ * updater gave up at a grid barrier, so that its slices are not the solution: call it
+ * after the stream of ps_updater_solve_device has been waited for.  Does not touch the
+ * device; the updater's next solve reports the same. */
+int ps_updater_check(ps_updater* u);
 
 /* ---- density (Updater::solve(data, q, qc, cc), include/Updater.h:57-58) */
 /* phi = cc * ds * sum_s c_s q[s] qc[len-1-s] with the weights of `rule`.

@@ -68,6 +68,10 @@ class _Updater:
         capi.check(lib().ps_updater_solve(self._h, capi.dptr(w), capi.dptr(qs), qs.shape[0]))
         return qs
 
+    def check(self):
+        """Raises if a solve on CUDA tensors, whose stream has been waited for, gave up."""
+        capi.check(lib().ps_updater_check(self._h))
+
     def __del__(self):
         h = getattr(self, "_h", None)
         if h:

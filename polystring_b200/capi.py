@@ -72,6 +72,7 @@ SIGNATURES = [
     ("ps_updater_destroy", None, [_vp]),
     ("ps_updater_solve", ctypes.c_int, [_vp, _dp, _dp, ctypes.c_int]),
     ("ps_updater_solve_device", ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
+    ("ps_updater_check", ctypes.c_int, [_vp]),
     ("ps_density_solve", ctypes.c_int, [ctypes.c_int, _dp, _dp, ctypes.c_int, ctypes.c_longlong,
                                         ctypes.c_double, ctypes.c_double, _dp]),
     ("ps_density_solve_device", ctypes.c_int, [ctypes.c_int, _vp, _vp, ctypes.c_int, ctypes.c_longlong,

@@ -267,7 +267,7 @@ void ModelAB::grad_w(const double* phiA_bar, const double* phiB_bar, double Q_ba
     PS_CUDA(cudaMemcpyAsync(pb.data(), phiB_.p, sizeof(double) * M_, cudaMemcpyDeviceToHost, st_));
     double Q = 0;
     PS_CUDA(cudaMemcpyAsync(&Q, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     double dot = 0.0;
     for (long i = 0; i < M_; i++) dot += phiA_bar[i] * pa[i] + phiB_bar[i] * pb[i];
     const double Qbar = Q_bar - dot / Q;
@@ -307,7 +307,7 @@ void ModelAB::grad_w(const double* phiA_bar, const double* phiB_bar, double Q_ba
     chain_->enqueue_adjoint(c, st_);
     PS_CUDA(cudaMemcpyAsync(gA, gA_.p, sizeof(double) * M_, cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaMemcpyAsync(gB, gB_.p, sizeof(double) * M_, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
 }
 
 void ModelAB::stress(double* dFdl) {
@@ -345,7 +345,7 @@ void ModelAB::stress(double* dFdl) {
     double Q = 0.0, dQ[3];
     PS_CUDA(cudaMemcpyAsync(&Q, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaMemcpyAsync(dQ, scal_.p + 16, sizeof(double) * 3, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     for (int i = 0; i < 3; i++) dFdl[i] = -dQ[i] / Q;
 }
 
@@ -418,7 +418,7 @@ void ModelAB::stress_checkpointed(int k, double* dFdl) {
     double Q = 0.0, dQl[3];
     PS_CUDA(cudaMemcpyAsync(&Q, dQ, sizeof(double), cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaMemcpyAsync(dQl, scal_.p + 16, sizeof(double) * 3, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     for (int i = 0; i < 3; i++) dFdl[i] = -dQl[i] / Q;
 }
 

@@ -338,7 +338,7 @@ void ModelAB::grad_w_sweep(const double* phiA_bar, const double* phiB_bar, doubl
     PS_CUDA(cudaGetLastError());
     PS_CUDA(cudaMemcpyAsync(gA, gA_.p, sizeof(double) * M_, cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaMemcpyAsync(gB, gB_.p, sizeof(double) * M_, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
 }
 
 void ModelAB::stress_sweep(double* dFdl) {
@@ -388,7 +388,7 @@ void ModelAB::stress_sweep(double* dFdl) {
     double Q = 0.0, dQ[3];
     PS_CUDA(cudaMemcpyAsync(&Q, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaMemcpyAsync(dQ, scal_.p + 16, sizeof(double) * 3, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     for (int i = 0; i < 3; i++) dFdl[i] = -dQ[i] / Q;
 }
 

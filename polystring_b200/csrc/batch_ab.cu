@@ -381,12 +381,12 @@ ModelABC& BatchAB::model_abc(int k) {
 }
 
 void BatchAB::set_fields(int k, const double* wA, const double* wB, bool device_ptrs) {
-    sync();
+    wait();
     model(k).set_fields(wA, wB, device_ptrs);
 }
 
 void BatchAB::set_fields_abc(int k, const double* const w[3], bool device_ptrs) {
-    sync();
+    wait();
     model_abc(k).set_fields(w, device_ptrs);
 }
 
@@ -429,10 +429,17 @@ double BatchAB::update_timed(int n) {
     PS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    sync();
     return ms;
 }
 
-void BatchAB::sync() { PS_CUDA(cudaStreamSynchronize(st_)); }
+void BatchAB::sync() {
+    wait();
+    for (auto* m : m_) m->check();
+    for (auto* m : t_) m->check();
+}
+
+void BatchAB::wait() { PS_CUDA(cudaStreamSynchronize(st_)); }
 
 double BatchAB::gridpoint_steps_per_iteration() const {
     double s = 0.0;

@@ -23,7 +23,7 @@ public:
     void update(int n);
     // update() between CUDA events on the batch stream; returns the device ms
     double update_timed(int n);
-    void sync();
+    void sync();   // and the members' check()
     int launches_per_iteration() const { return launches_; }
     int launches_per_propagate() const { return launches_prop_; }
     // sum over solves of 2 Ns M: gridpoint contour steps of one iteration
@@ -59,6 +59,7 @@ private:
     const RealSweep* sweep_of(int k) const;
     void add_chunk(const std::vector<int>& ks, const std::vector<int>& per, int cluster);
     void build_sweeps(const std::vector<int>& members);
+    void wait();
     void release();
     void enqueue_iteration();
     std::vector<ModelAB*> m_;

@@ -115,6 +115,13 @@ int ps_updater_solve_device(ps_updater* u, const double* w, double* qs, int len,
     });
 }
 
+int ps_updater_check(ps_updater* u) {
+    return guarded([&] {
+        if (!u) throw Error(PS_ERR_INVALID, "null handle");
+        u->ctx->check();
+    });
+}
+
 int ps_density_solve_device(int rule, const double* q, const double* qc, int len, long long M, double ds, double cc,
                             double* phi, void* stream) {
     return guarded([&] {
@@ -249,7 +256,7 @@ int ps_model_abc_get(ps_model_abc* m, int which, double* out) {
 int ps_model_abc_synchronize(ps_model_abc* m) {
     return guarded([&] {
         if (!m) throw Error(PS_ERR_INVALID, "null handle");
-        PS_CUDA(cudaStreamSynchronize(m->ctx->stream()));
+        m->ctx->sync();
     });
 }
 

@@ -520,6 +520,7 @@ void ModelAB::set_fields(const double* wA, const double* wB, bool dev) {
     if (p_.scft == 1) init_anderson(wA, wB, dev);
     launch_factors(wA_.p, wB_.p, M_, dsA_, dsB_, eFA_.p, eHA_.p, eFB_.p, eHB_.p, 1, 0, st_);
     PS_CUDA(cudaStreamSynchronize(st_));
+    if (real_) real_->reset(st_);
     iter_ = 0;
     fields_set_ = true;
     forward_done_ = false;
@@ -607,6 +608,7 @@ static cudaGraphExec_t capture(cudaStream_t st, F&& body) {
 
 void ModelAB::ensure_graphs() {
     if (!fields_set_) throw Error(-6, "fields are not set");
+    check();
     if (!gprop_) gprop_ = capture(st_, [&] { enqueue_propagate(); });
     if (!gpost_) gpost_ = capture(st_, [&] { enqueue_post(); });
 }
@@ -636,6 +638,7 @@ double ModelAB::update_timed(int n, double* prop_ms) {
     PS_CUDA(cudaEventRecord(ev[2 * n + 1], st_));
     iter_ += n;
     PS_CUDA(cudaStreamSynchronize(st_));
+    check();
     double total = 0.0;
     for (int i = 0; i < n; i++) {
         float ms = 0.f;
@@ -654,13 +657,16 @@ void ModelAB::propagate(int n) {
     for (int i = 0; i < n; i++) PS_CUDA(cudaGraphLaunch(gprop_, st_));
 }
 
-void ModelAB::sync() { PS_CUDA(cudaStreamSynchronize(st_)); }
+void ModelAB::sync() {
+    PS_CUDA(cudaStreamSynchronize(st_));
+    check();
+}
 
 double ModelAB::Q() {
     if (iter_ == 0 && !forward_done_) throw Error(-6, "no iteration has run");
     double q = 0;
     PS_CUDA(cudaMemcpyAsync(&q, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     return q;
 }
 
@@ -669,7 +675,7 @@ void ModelAB::H(double* H, double* Hw, double* Hs) {
     launch_Hw(phiA_.p, phiB_.p, wA_.p, wB_.p, M_, p_.chiN, p_.lamYita, p_.compressible, partial_.p, scal_.p + 1, st_);
     double h[2];
     PS_CUDA(cudaMemcpyAsync(h, scal_.p, sizeof(double) * 2, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     *Hw = h[1];
     *Hs = -log(h[0]);
     *H = *Hw + *Hs;
@@ -686,14 +692,14 @@ double ModelAB::residual() {
                            hwB_.p + (long)pos * M_, M_, partial_.p, scal_.p + 2, st_);
         double e[4];
         PS_CUDA(cudaMemcpyAsync(e, scal_.p + 2, sizeof(double) * 4, cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
+        sync();
         return sqrt((e[0] + e[2]) / (e[1] + e[3]));
     }
     launch_residual_em(phiA_.p, phiB_.p, wA_.p, wB_.p, yita_.p, M_, p_.chiN, p_.lamYita, p_.compressible,
                        partial_.p, scal_.p + 2, st_);
     double v[8];
     PS_CUDA(cudaMemcpyAsync(v, scal_.p + 2, sizeof(double) * 8, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     double res = 0.0;
     res += v[0] / (v[1] + v[2]);
     res += v[3] / (v[4] + v[5]);
@@ -704,18 +710,6 @@ double ModelAB::residual() {
         res /= 2.0;
     }
     return res;
-}
-
-int ModelAB::status() {
-    int st = 0;
-    if (axs_) {
-        AXState s;
-        PS_CUDA(cudaMemcpyAsync(&s, axs_, sizeof(AXState), cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
-        st |= s.status;
-    }
-    if (real_ && real_->error(st_)) st |= 2;
-    return st;
 }
 
 double* ModelAB::device_ptr(int which) {
@@ -740,7 +734,7 @@ void ModelAB::get(int which, double* out, bool device_dst) {
     double* src = device_ptr(which);
     PS_CUDA(cudaMemcpyAsync(out, src, sizeof(double) * count,
                             device_dst ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
 }
 
 // ---------------------------------------------------------------------------
@@ -793,6 +787,7 @@ UpdaterCtx* UpdaterCtx::clone() const { return new UpdaterCtx(scheme_, cell_, Lx
 
 void UpdaterCtx::solve_device(const double* w, double* qs, int len, cudaStream_t st) {
     if (len < 1) throw Error(-1, "propagator length must be at least 1");
+    check();   // an earlier solve's
     if (len == 1) return;
     if (!st) st = st_;
     if (scheme_ == SCHEME_ETDRK4) {
@@ -826,7 +821,13 @@ void UpdaterCtx::solve_host(const double* w, double* qs, int len) {
         PS_CUDA(cudaMemcpyAsync(qs + M_, dqs_.p + M_, sizeof(double) * (size_t)(len - 1) * M_,
                                 cudaMemcpyDeviceToHost, st_));
     PS_CUDA(cudaStreamSynchronize(st_));
-    if (real_ && real_->error(st_)) throw Error(-3, "the propagator sweep reported a barrier timeout");
+    check();
+}
+
+void UpdaterCtx::check() {
+    if (!real_ || !real_->failed()) return;
+    real_->reset(st_);
+    throw Error(-3, "a propagator sweep gave up at a grid barrier (its CTAs were not all running)");
 }
 
 }  // namespace ps

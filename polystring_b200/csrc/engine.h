@@ -185,7 +185,9 @@ public:
     long M() const { return M_; }
     int Ns() const { return Ns_; }
     long iterations() const { return iter_; }
-    int status();
+    // throws if a sweep of this solve that has ended gave up at a barrier; so do the
+    // calls that wait for its results, until fields are set again
+    void check() const { if (real_) real_->check(); }
     const ModelABParams& params() const { return p_; }
     bool persistent_sweep() const { return real_ != nullptr; }
     const RealSweep* sweep() const { return real_; }
@@ -287,7 +289,8 @@ public:
     double residual();
     // 0..2 wA, wB, wC; 3..5 phiA, phiB, phiC; 6 yita
     void get(int which, double* out, bool device_dst);
-    int status();
+    void sync();
+    void check() const { if (real_) real_->check(); }   // as ModelAB's
     long M() const { return M_; }
     int Ns() const { return Ns_; }
     int L(int x) const { return L_[x]; }
@@ -332,6 +335,8 @@ public:
     ~UpdaterCtx();
     UpdaterCtx* clone() const;
     void solve_device(const double* w, double* qs, int len, cudaStream_t st);
+    // throws, once, if a solve that has ended gave up at a barrier
+    void check();
     void solve_host(const double* w, double* qs, int len);
     int scheme() const { return scheme_; }
 

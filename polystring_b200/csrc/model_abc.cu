@@ -127,6 +127,7 @@ void ModelABC::set_fields(const double* const w[3], bool dev) {
     launch_factors(w_[0].p, w_[1].p, M_, ds_[0], ds_[1], eF_[0].p, eH_[0].p, eF_[1].p, eH_[1].p, 1, 0, st_);
     launch_factors(w_[2].p, w_[2].p, M_, ds_[2], ds_[2], eF_[2].p, eH_[2].p, eF_[2].p, eH_[2].p, 1, 0, st_);
     PS_CUDA(cudaStreamSynchronize(st_));
+    if (real_) real_->reset(st_);
     iter_ = 0;
     fields_set_ = true;
 }
@@ -196,6 +197,7 @@ void ModelABC::enqueue_iteration(cudaStream_t st) {
 
 void ModelABC::update(int n) {
     if (!fields_set_) throw Error(-6, "fields are not set");
+    check();
     if (!graph_) {
         PS_CUDA(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
         cudaGraph_t g = nullptr;
@@ -219,7 +221,7 @@ double ModelABC::Q() {
     if (iter_ == 0) throw Error(-6, "no iteration has run");
     double q = 0;
     PS_CUDA(cudaMemcpyAsync(&q, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     return q;
 }
 
@@ -230,7 +232,7 @@ void ModelABC::H(double* H, double* Hw, double* Hs) {
     launch_Hw_abc(phi, w, p_.chi, M_, partial_.p, scal_.p + 1, st_);
     double h[2];
     PS_CUDA(cudaMemcpyAsync(h, scal_.p, sizeof(double) * 2, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     *Hw = h[1];
     *Hs = -log(h[0]);
     *H = *Hw + *Hs;
@@ -252,7 +254,7 @@ double ModelABC::residual() {
         launch_residual_ax_abc(d, w, M_, partial_.p, scal_.p + 2, st_);
         double e[6];
         PS_CUDA(cudaMemcpyAsync(e, scal_.p + 2, sizeof(double) * 6, cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
+        sync();
         return sqrt((e[0] + e[2] + e[4]) / (e[1] + e[3] + e[5]));
     }
     const double* phi[3] = {phi_[0].p, phi_[1].p, phi_[2].p};
@@ -260,7 +262,7 @@ double ModelABC::residual() {
     launch_residual_em_abc(phi, w, yita_.p, p_.chi, M_, partial_.p, scal_.p + 2, st_);
     double v[11];
     PS_CUDA(cudaMemcpyAsync(v, scal_.p + 2, sizeof(double) * 11, cudaMemcpyDeviceToHost, st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
     double res = 0.0;
     for (int x = 0; x < 3; x++) res += v[3 * x] / (v[3 * x + 1] + v[3 * x + 2]);
     res += v[9] / (1.0 + v[10]);
@@ -275,19 +277,12 @@ void ModelABC::get(int which, double* out, bool device_dst) {
     else throw Error(-1, "unknown field");
     PS_CUDA(cudaMemcpyAsync(out, src, sizeof(double) * M_, device_dst ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                             st_));
-    PS_CUDA(cudaStreamSynchronize(st_));
+    sync();
 }
 
-int ModelABC::status() {
-    int st = 0;
-    if (axs_) {
-        AXState s;
-        PS_CUDA(cudaMemcpyAsync(&s, axs_, sizeof(AXState), cudaMemcpyDeviceToHost, st_));
-        PS_CUDA(cudaStreamSynchronize(st_));
-        st |= s.status;
-    }
-    if (real_ && real_->error(st_)) st |= 2;
-    return st;
+void ModelABC::sync() {
+    PS_CUDA(cudaStreamSynchronize(st_));
+    check();
 }
 
 }  // namespace ps

@@ -32,9 +32,10 @@
 // CTAs an SM gain nothing alone (19 to 20 us at 64^3), a barrier a field costs 10.2 us
 // at 32^3, two columns a lane 19.1 at 64^3.
 //
-// Barriers count arrivals per solve with a bounded spin; the launch is
-// cooperative, so all CTAs are resident.  On a timeout the CTA raises the error
-// flag, every CTA of the solve sees it and returns, and the host reports it.
+// Barriers (sweep_barrier.cuh) count arrivals per chain with a bounded spin; the launch
+// is cooperative, so all CTAs are resident.  On a timeout the CTA raises the error
+// flag, every CTA of the solve sees it and returns, and the host finds a word in its
+// own memory set: RealSweep::check.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -48,41 +49,14 @@
 #include "fft_core.cuh"
 #include "real_line.cuh"
 #include "real_sweep.h"
+#include "sweep_barrier.cuh"
 
 namespace ps {
 
 namespace {
 
-constexpr long long kSpinLimit = 20000000;   // polls before a barrier gives up
 constexpr int kNT = 256;                     // threads a CTA
 constexpr size_t kSmemLimit = 227 * 1024 - 1024;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_release_add(unsigned* p, unsigned v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Barrier over the CTAs of one solve.  Returns false when the sweep must stop.
-__device__ __forceinline__ bool solve_barrier(unsigned* count, int* err, unsigned target) {
-    __shared__ int stop;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int s = 0;
-        red_release_add(count, 1u);
-        long long spins = 0;
-        while (ld_acquire(count) < target) {
-            if ((spins & 63) == 63 && *((volatile int*)err)) { s = 1; break; }
-            if (++spins > kSpinLimit) { atomicExch(err, 2); s = 1; break; }
-        }
-        stop = s;
-    }
-    __syncthreads();
-    return stop == 0;
-}
 
 // row pitch of a slab in shared memory: 4 mod 8 doubles, so that the 4 rows x 4
 // consecutive values of a half warp fall in different banks, by rows and by
@@ -407,7 +381,7 @@ __global__ void __launch_bounds__(kNT, ONE ? 1 : 2) real_sweep_kernel(const __gr
         if (t >= 0) {
             run_x<ONE>(p, frx, xcache, ch, t, w, nw);
             target += ncta;
-            if (!solve_barrier(bar, p.err, target)) return;
+            if (!chain_barrier(p, bar, target)) return;
         }
         for (int slab = cta; slab < p.Lx; slab += ncta) {
             if (t >= 0) {
@@ -423,7 +397,7 @@ __global__ void __launch_bounds__(kNT, ONE ? 1 : 2) real_sweep_kernel(const __gr
         }
         if (t + 1 < p.Ns) {
             target += ncta;
-            if (!solve_barrier(bar, p.err, target)) return;
+            if (!chain_barrier(p, bar, target)) return;
         }
     }
 }
@@ -549,6 +523,39 @@ void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool one, 
 // ---------------------------------------------------------------------------
 // RealSweep
 // ---------------------------------------------------------------------------
+// Words of pinned host memory that kernels of every device can write, one a sweep
+// alive.  A sweep returns its word for the next; a page of them (of 1024) stays for the
+// process: a page each would cost every construction 2 ms.
+namespace {
+class Notices {
+public:
+    int* take() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (free_.empty()) {
+            int* page = nullptr;
+            PS_CUDA(cudaHostAlloc(&page, 1024 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+            for (int i = 1023; i >= 0; i--) free_.push_back(page + i);
+        }
+        int* w = free_.back();
+        free_.pop_back();
+        *w = 0;
+        return w;
+    }
+    void give(int* w) {
+        std::lock_guard<std::mutex> lock(mu_);
+        free_.push_back(w);
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<int*> free_;
+};
+Notices& notices() {
+    static Notices* n = new Notices;   // objects may be destroyed after statics are
+    return *n;
+}
+}  // namespace
+
 bool RealSweep::supported(int Lx, int Ly, int Lz) {
     if (Ly == 1 && Lz == 1) return line_sweep_supported(Lx);
     if (Lz == 1) return plane_sweep_supported(Lx, Ly) || tile_sweep_supported(Lx, Ly);
@@ -584,12 +591,18 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     PS_CUDA(cudaMemcpy(frag_, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
     PS_CUDA(cudaMalloc(&bar_, 33 * sizeof(unsigned)));
     PS_CUDA(cudaMemset(bar_, 0, 33 * sizeof(unsigned)));
+    if (dim_ == 3 || (tile_ && !cluster_)) {
+        notice_ = notices().take();
+    }
+    const char* polls = getenv("PS_B200_BARRIER_POLLS");
+    polls_ = polls ? std::max(0, atoi(polls)) : kBarrierPolls;
 }
 
 RealSweep::~RealSweep() {
     cudaFree(work_);
     cudaFree(frag_);
     cudaFree(bar_);
+    if (notice_) notices().give(notice_);
 }
 
 RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
@@ -603,6 +616,8 @@ RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
     p.nfrag = nfrag_;
     p.bar = bar_;
     p.err = reinterpret_cast<int*>(bar_ + 32);
+    p.notice = notice_;
+    p.polls = polls_;
     p.Lx = n_[0]; p.Ly = n_[1]; p.Lz = n_[2];
     p.Ns = Ns;
     p.nl = nl_;
@@ -615,16 +630,21 @@ void RealSweep::enqueue(const RealProblem& p, cudaStream_t st) const {
     if (dim_ == 1) return line_sweep_launch(p, st);
     if (dim_ == 2 && !tile_) return plane_sweep_launch(p, st);
     if (cluster_) return tile_cluster_launch(p, cluster_, st);
-    PS_CUDA(cudaMemsetAsync(bar_, 0, 32 * sizeof(unsigned), st));
+    PS_CUDA(cudaMemsetAsync(bar_, 0, 33 * sizeof(unsigned), st));
     if (tile_) return tile_sweep_launch(p, ncta_, st);
     real_sweep_launch(p, ncta_, st);
 }
 
-int RealSweep::error(cudaStream_t st) const {
-    int e = 0;
-    PS_CUDA(cudaMemcpyAsync(&e, bar_ + 32, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PS_CUDA(cudaStreamSynchronize(st));
-    return e;
+bool RealSweep::failed() const { return notice_ && *((volatile int*)notice_); }
+
+void RealSweep::check() const {
+    if (failed()) throw Error(-3, "a propagator sweep gave up at a grid barrier (its CTAs were not all running)");
+}
+
+void RealSweep::reset(cudaStream_t st) {
+    if (!failed()) return;
+    PS_CUDA(cudaMemsetAsync(bar_ + 32, 0, sizeof(unsigned), st));
+    *((volatile int*)notice_) = 0;
 }
 
 void RealSweep::tune(const RealProblem& p0, cudaStream_t st) {
@@ -675,7 +695,7 @@ void RealSweep::tune(const RealProblem& p0, cudaStream_t st) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (error(st)) throw Error(-3, "persistent sweep reported an error while it was timed");
+    check();
     variant_ = pick;
     if (n > 0 && n < (int)sizeof(line))
         std::snprintf(line + n, sizeof(line) - n, " -> %d\n", real_sweep_columns(pick));

@@ -33,7 +33,9 @@ struct RealProblem {
     const double* frag;   // the axes' operators (full step, half step): B fragments, or parts (1D; 2D axes past 64)
     int fo[3], nfrag;     // where each axis's start (axes of equal length and spacing share), doubles in all
     unsigned* bar;        // barrier counters (one a chain, 16 words apart), zeroed before the launch
-    int* err;             // nonzero after a barrier timeout
+    int* err;             // nonzero after a barrier timeout, for the chains' CTAs
+    int* notice;          // the same in host memory
+    int polls;            // after which a barrier gives up
     int Lx, Ly, Lz, Ns, nl;
     int os2;              // second-order splitting: full steps only
     int xcols;            // columns of an x-pass task (a multiple of 8)
@@ -99,6 +101,10 @@ void tile_string_launch(const RealProblem* d, int n, size_t smem, cudaStream_t s
 bool line_sweep_supported(int Lx);
 void line_sweep_launch(const RealProblem& p, cudaStream_t st);
 
+// polls before a barrier gives up, some ten seconds (PS_B200_BARRIER_POLLS=n: n, from
+// the sweep's construction on)
+constexpr int kBarrierPolls = 20000000;
+
 // The work fields, operators and barrier words of one solve's sweep.
 class RealSweep {
 public:
@@ -118,7 +124,11 @@ public:
     void enqueue(const RealProblem& p, cudaStream_t st) const;
     bool tiled() const { return tile_; }   // 2D, the chains in tiles of lines
     int cluster() const { return cluster_; }
-    int error(cudaStream_t st) const;   // barrier error flag (synchronises)
+    // whether a sweep that has ended gave up at a barrier (the fields it wrote are not
+    // the chains'), throwing if so, and a new start after that
+    bool failed() const;
+    void check() const;
+    void reset(cudaStream_t st);
 
 private:
     int n_[3], dim_, nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
@@ -126,6 +136,8 @@ private:
     int cluster_ = 0;   // CTAs of a chain's cluster (0: chains over the grid)
     double *work_ = nullptr, *frag_ = nullptr;
     unsigned* bar_ = nullptr;   // 32 words, then the error flag
+    int* notice_ = nullptr;     // the error flag's copy in host memory (forms with barriers in memory)
+    int polls_ = kBarrierPolls;
 };
 
 }  // namespace ps

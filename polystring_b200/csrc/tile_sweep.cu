@@ -40,6 +40,7 @@
 #include "fft_core.cuh"
 #include "real_line.cuh"
 #include "real_sweep.h"
+#include "sweep_barrier.cuh"
 
 namespace ps {
 
@@ -47,35 +48,7 @@ namespace {
 
 constexpr int kNT = 256;      // threads of a CTA of the grid form
 constexpr int kStringNT = 128;   // and of a string's clusters: three CTAs an SM
-constexpr long long kSpinLimit = 20000000;   // polls before a barrier gives up
 constexpr size_t kSmemLimit = 227 * 1024 - 1024;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_release_add(unsigned* p, unsigned v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Barrier over the CTAs of one chain.  Returns false when the sweep must stop.
-__device__ __forceinline__ bool chain_barrier(unsigned* count, int* err, unsigned target) {
-    __shared__ int stop;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int s = 0;
-        red_release_add(count, 1u);
-        long long spins = 0;
-        while (ld_acquire(count) < target) {
-            if ((spins & 63) == 63 && *((volatile int*)err)) { s = 1; break; }
-            if (++spins > kSpinLimit) { atomicExch(err, 2); s = 1; break; }
-        }
-        stop = s;
-    }
-    __syncthreads();
-    return stop == 0;
-}
 
 // barrier over the cluster's CTAs, with their writes to global memory
 __device__ __forceinline__ void cluster_barrier() {
@@ -553,7 +526,7 @@ __global__ void __launch_bounds__(NT, PER_SM) tile_sweep_kernel(const __grid_con
             return true;
         }
         target += ncta;
-        return chain_barrier(bar, p.err, target);
+        return chain_barrier(p, bar, target);
     };
     for (int t = -1; t < p.Ns; t++) {
         if (t >= 0) {
