@@ -18,11 +18,13 @@
 // head.  dD/dl_i = h (8 pi^2 / l_i^3) R_i D with the line operator
 // R_i = F^-1 r_i^2 F of axis i, so
 //
-//   lambda' (dA/dl_i) q = h 8 pi^2 / l_i^3 [ 2/3 ((e' lambda) . R_i (D' e' S' q) + (e D' e' lambda) . R_i (D' e' q))
+//   lambda' (dA/dl_i) q = h 8 pi^2 / l_i^3 [ 2/3 ((D' e' lambda) . R_i (e D' e' q) + (e D' e' lambda) . R_i (D' e' q))
 //                                           - 1/3 (e lambda) . R_i (D e q) ]
 //
 // with e = e^{-w ds/2}, e' = e^{-w ds/4}: three line operators an axis and step,
-// all steps at once.
+// all steps at once.  (The first term is (e' lambda) . R_i (D' e' S' q): D' is
+// symmetric, commutes with R_i, and e' S' q = e D' e' q.  So only kept fields enter, and
+// no quotient by e', which is zero where w is large or infinite.)
 //
 // 48^3, Ns 128 (B200): the reverse sweeps took about 80 us a step and chain on
 // line passes (gradient 33.5 ms, stress 21.9 ms a call with the forward map).
@@ -133,9 +135,9 @@ __global__ void __launch_bounds__(kT) grad_sum_kernel(const double* partial, con
 __device__ __forceinline__ long line_base(long l, int N, long st) { return l / st * N * st + l % st; }
 
 struct StressArgs {
-    const double *q, *qhalf, *qfull;   // forward chain: slices, kept fields
-    const double *c, *chalf;           // complementary chain
-    const double *eF[2], *eH[2];
+    const double *qhalf, *qfull;       // forward chain: kept fields
+    const double *c, *chalf;           // complementary chain: slices, kept fields
+    const double* eF[2];
     const double* frag;                // R_i
     double scale[2];                   // 8 pi^2 / l^3 times the block's ds
     double* partial;                   // [cta][3], entry `axis`
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(kT, 2) stress_axis_kernel(const StressArgs a) 
         const bool ok = l < a.nlines;
         const long base = line_base(ok ? l : l - g, N, a.st), now = (long)t * a.M + base;
         const long lam = (long)(a.Ns - 1 - t) * a.M + base;   // lambda[t + 1]
-        const double *eF = a.eF[blk] + base, *eH = a.eH[blk] + base;
+        const double* eF = a.eF[blk] + base;
         double part = 0.0;
 #pragma unroll 1
         for (int k = 0; k < 3; k++) {
@@ -172,9 +174,7 @@ __global__ void __launch_bounds__(kT, 2) stress_axis_kernel(const StressArgs a) 
                     double v = 0.0;
                     if (R::WHOLE || o < R::O) {
                         const long n = R::point(i, o) * a.st;
-                        if (k == 0) v = a.qfull[now + n];
-                        else if (k == 2) v = a.qhalf[now + n];
-                        else v = (3.0 * a.q[now + a.M + n] + eF[n] * a.qfull[now + n]) / (4.0 * eH[n]);
+                        v = k == 0 ? a.qfull[now + n] : k == 1 ? eF[n] * a.qhalf[now + n] : a.qhalf[now + n];
                     }
                     x[4 * s + i] = v;
                 }
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kT, 2) stress_axis_kernel(const StressArgs a) 
                     const int o = j + 4 * s;
                     if (R::WHOLE || o < R::O) {
                         const long n = R::point(i, o) * a.st;
-                        const double y = k == 0 ? eF[n] * a.c[lam + n] : k == 1 ? eH[n] * a.c[lam + n]
+                        const double y = k == 0 ? eF[n] * a.c[lam + n] : k == 1 ? a.chalf[lam + n]
                                                                                 : eF[n] * a.chalf[lam + n];
                         d += x[4 * s + i] * y;
                     }
@@ -367,9 +367,9 @@ void ModelAB::stress_sweep(double* dFdl) {
         if (n[ax] == 1) continue;
         const double l = p_.cell.l[ax], c = l > 0 ? 8.0 * PI * PI / (l * l * l) : 0.0;
         StressArgs a{};
-        a.q = hf_.p; a.qhalf = kept_[0].p; a.qfull = kept_[1].p;
+        a.qhalf = kept_[0].p; a.qfull = kept_[1].p;
         a.c = hc_.p; a.chalf = kept_[2].p;
-        a.eF[0] = eFA_.p; a.eF[1] = eFB_.p; a.eH[0] = eHA_.p; a.eH[1] = eHB_.p;
+        a.eF[0] = eFA_.p; a.eF[1] = eFB_.p;
         a.frag = sfrag_.p + sfo_[ax];
         a.scale[0] = c * dsA_; a.scale[1] = c * dsB_;
         a.partial = spart_.p;
