@@ -214,7 +214,11 @@ int ps_model_ab_forward(ps_model_ab* m);
  * reference, which has no derivatives): with the current fields, writes
  * dL/dwA and dL/dwB (M doubles each, host memory) for
  * L = sum_r (dL_dphiA phiA + dL_dphiB phiB) + dL_dQ Q, exact for the
- * discrete RQM4 chain and contour rule; the forward map is re-evaluated. */
+ * discrete RQM4 chain and contour rule; the forward map is re-evaluated.
+ * On grids with a persistent sweep the first call allocates 10 Ns M doubles for
+ * intermediate fields of every step (ps_model_ab_stress: 4 Ns M of them), which the
+ * model keeps, if that leaves a sixteenth of the device's memory free; else, and on
+ * other grids, slower line passes need only a few fields. */
 int ps_model_ab_grad_w(ps_model_ab* m, const double* dL_dphiA, const double* dL_dphiB, double dL_dQ,
                        double* dL_dwA, double* dL_dwB);
 /* Cell stress d(-ln Q)/dl_i at the current fields for the three cell

@@ -241,13 +241,14 @@ void ModelAB::adjoint_weights(std::vector<double>& wAf, std::vector<double>& wBf
 }
 
 void ModelAB::ensure_adjoint_buffers(bool spec) {
-    if (lam_.n == 0) {
+    // the last one of each group tells that all are there
+    if (pbB_.n == 0) {
         lam_.alloc(2 * (size_t)M_);
         gA_.alloc(M_); gB_.alloc(M_);
-        pbA_.alloc(M_); pbB_.alloc(M_);
         chain_->prepare_adjoint();
+        pbA_.alloc(M_); pbB_.alloc(M_);
     }
-    if (spec && spec_.n == 0) {
+    if (spec && stress_part_.n == 0) {
         spec_.alloc(6 * (size_t)M_);
         stress_part_.alloc((size_t)Ns_ * 148 * 3);
     }
@@ -258,6 +259,7 @@ void ModelAB::grad_w(const double* phiA_bar, const double* phiB_bar, double Q_ba
     if (p_.mde != 0) throw Error(-2, "the adjoint is provided for RQM4");
     ensure_adjoint_buffers(false);
     if (sweep_adjoint(true)) return grad_w_sweep(phiA_bar, phiB_bar, Q_bar, gA, gB);
+    if (real_) chain_->autotune(st_);   // models without a sweep did when they were made
     forward_only();
     // pbar = phi_bar / Q; Qbar_total = Q_bar - (1/Q) sum(phi_bar phi)
     PS_CUDA(cudaMemcpyAsync(pbA_.p, phiA_bar, sizeof(double) * M_, cudaMemcpyHostToDevice, st_));
@@ -315,6 +317,7 @@ void ModelAB::stress(double* dFdl) {
     if (p_.mde != 0) throw Error(-2, "the adjoint is provided for RQM4");
     if (sweep_adjoint(false)) return stress_sweep(dFdl);
     ensure_adjoint_buffers(true);
+    if (real_) chain_->autotune(st_);
     forward_only();
     PS_CUDA(cudaMemsetAsync(gA_.p, 0, sizeof(double) * M_, st_));
     PS_CUDA(cudaMemsetAsync(gB_.p, 0, sizeof(double) * M_, st_));
@@ -356,10 +359,10 @@ void ModelAB::stress_checkpointed(int k, double* dFdl) {
     if (k > Ns_) k = Ns_;
     const int nseg = (Ns_ + k - 1) / k;
     ensure_adjoint_buffers(true);
-    if (real_) chain_->autotune(st_);   // models without a sweep did when they were made
+    if (real_) chain_->autotune(st_);
     ck_.alloc((size_t)nseg * M_);
     seg_.alloc((size_t)(k + 1) * M_);
-    if (zero_.n == 0) {
+    if (scratch_.n == 0) {
         zero_.alloc(M_);
         scratch_.alloc(M_);
         launch_fill(zero_.p, M_, 0.0, st_);

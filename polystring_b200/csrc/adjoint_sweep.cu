@@ -28,7 +28,10 @@
 //
 // 48^3, Ns 128 (B200): the reverse sweeps took about 80 us a step and chain on
 // line passes (gradient 33.5 ms, stress 21.9 ms a call with the forward map).
+#include <algorithm>
 #include <cmath>
+#include <utility>
+#include <vector>
 
 #include "engine.h"
 #include "field_kernels.h"
@@ -87,12 +90,11 @@ struct GradChain {
     const double *q, *lam, *qhalf, *qfull, *lhalf, *lfull;
     const double *src_w[2], *src_o;
 };
-struct Chunk { int chain, blk, t0, t1; };
 struct GradArgs {
     GradChain c[2];
     const double *eF[2], *pA, *pB;
     double ds[2];
-    const Chunk* chunk;
+    const AdjointChunk* chunk;
     double* partial;
     long M;
     int Ns;
@@ -102,7 +104,7 @@ struct GradArgs {
 __global__ void __launch_bounds__(kT) grad_kernel(const GradArgs a) {
     const long i = (long)blockIdx.x * kT + threadIdx.x;
     if (i >= a.M) return;
-    const Chunk k = a.chunk[blockIdx.y];
+    const AdjointChunk k = a.chunk[blockIdx.y];
     const GradChain& c = a.c[k.chain];
     const long M = a.M;
     const double e = a.eF[k.blk][i], pA = a.pA[i], pB = a.pB[i], ds = a.ds[k.blk];
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(kT) grad_kernel(const GradArgs a) {
     }
     a.partial[(long)blockIdx.y * M + i] = acc;
 }
-__global__ void __launch_bounds__(kT) grad_sum_kernel(const double* partial, const Chunk* chunk, int n, long M,
+__global__ void __launch_bounds__(kT) grad_sum_kernel(const double* partial, const AdjointChunk* chunk, int n, long M,
                                                       double* gA, double* gB) {
     const long i = (long)blockIdx.x * kT + threadIdx.x;
     if (i >= M) return;
@@ -231,28 +233,47 @@ void stress_launch(const StressArgs& a, cudaStream_t st) {
 // the grid has no sweep that keeps them (one with a single axis longer than a point,
 // in a cell of any dimension, has not) or the device has no room: the line passes
 // serve then, or refuse the grid.
+// The buffers stay with the model.  They leave a sixteenth of the device's memory free,
+// for others and for the line passes' own.
 bool ModelAB::sweep_adjoint(bool grad) {
     if (!real_ || chain_->plan().naxes < 2) return false;
     // the stress keeps an axis's operator in shared memory: 36 KB at 128 points, 250 KB at 352
     if (!grad && (p_.Lx > 128 || p_.Ly > 128 || p_.Lz > 128)) return false;
     const size_t n = (size_t)Ns_ * M_;
-    try {
-        for (DevBuf* b : {&kept_[0], &kept_[1], &kept_[2], &kept_[3]})
-            if (b->n == 0) b->alloc(n);
-        if (grad) {
-            for (DevBuf* b : {&lkept_[0], &lkept_[1], &lkept_[2], &lkept_[3]})
-                if (b->n == 0) b->alloc(n);
-            for (DevBuf* b : {&lamh_[0], &lamh_[1]})
-                if (b->n == 0) b->alloc(n + M_);
-        }
-    } catch (const Error&) {
-        cudaGetLastError();   // out of memory is not an error of this call
-        for (DevBuf& b : kept_) b.release();
-        for (DevBuf& b : lkept_) b.release();
-        for (DevBuf& b : lamh_) b.release();
-        return false;
+    std::vector<std::pair<DevBuf*, size_t>> missing;
+    size_t need = 0;
+    auto want = [&](DevBuf& b, size_t count) {
+        if (b.n > 0) return;
+        missing.push_back({&b, count});
+        need += sizeof(double) * count;
+    };
+    for (DevBuf& b : kept_) want(b, n);
+    if (grad) {
+        for (DevBuf& b : lkept_) want(b, n);
+        for (DevBuf& b : lamh_) want(b, n + M_);
+        want(gpart_, adjoint_chunks().size() * (size_t)M_);
     }
-    return true;
+    if (missing.empty()) return true;
+    size_t free = 0, total = 0;
+    PS_CUDA(cudaMemGetInfo(&free, &total));
+    bool room = need + total / 16 <= free;
+    for (size_t i = 0; room && i < missing.size(); i++) room = missing[i].first->try_alloc(missing[i].second);
+    if (!room)   // the stress's, where only the gradient's do not fit, stay
+        for (auto& m : missing) m.first->release();
+    return room;
+}
+
+// steps of both chains in chunks of one block each
+std::vector<AdjointChunk> ModelAB::adjoint_chunks() const {
+    std::vector<AdjointChunk> ch;
+    auto add = [&](int chain, int blk, int t0, int t1) {
+        for (int t = t0; t < t1; t += kChunk) ch.push_back({chain, blk, t, std::min(t + kChunk, t1)});
+    };
+    add(0, 0, 0, LA_);
+    add(0, 1, LA_, Ns_);
+    add(1, 1, 0, LB_);
+    add(1, 0, LB_, Ns_);
+    return ch;
 }
 
 // forward_only() with the kept fields
@@ -272,14 +293,7 @@ void ModelAB::grad_w_sweep(const double* phiA_bar, const double* phiB_bar, doubl
     std::vector<double> wAf, wBf;
     adjoint_weights(wAf, wBf);
     if (adj_chunks_ == 0) {
-        std::vector<Chunk> ch;
-        auto add = [&](int chain, int blk, int t0, int t1) {
-            for (int t = t0; t < t1; t += kChunk) ch.push_back({chain, blk, t, std::min(t + kChunk, t1)});
-        };
-        add(0, 0, 0, LA_);
-        add(0, 1, LA_, Ns_);
-        add(1, 1, 0, LB_);
-        add(1, 0, LB_, Ns_);
+        const std::vector<AdjointChunk> ch = adjoint_chunks();
         std::vector<double> w;
         for (int s = 0; s <= Ns_; s++) w.push_back(wAf[Ns_ - s]);
         for (int s = 0; s <= Ns_; s++) w.push_back(wBf[Ns_ - s]);
@@ -287,9 +301,8 @@ void ModelAB::grad_w_sweep(const double* phiA_bar, const double* phiB_bar, doubl
         w.insert(w.end(), wBf.begin(), wBf.end());
         srcw_.alloc(w.size());
         PS_CUDA(cudaMemcpy(srcw_.p, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice));
-        chunks_.alloc((sizeof(Chunk) * ch.size() + 7) / 8);
-        PS_CUDA(cudaMemcpy(chunks_.p, ch.data(), sizeof(Chunk) * ch.size(), cudaMemcpyHostToDevice));
-        gpart_.alloc(ch.size() * (size_t)M_);
+        chunks_.alloc((sizeof(AdjointChunk) * ch.size() + 7) / 8);
+        PS_CUDA(cudaMemcpy(chunks_.p, ch.data(), sizeof(AdjointChunk) * ch.size(), cudaMemcpyHostToDevice));
         adj_chunks_ = (int)ch.size();
     }
     PS_CUDA(cudaMemcpyAsync(pbA_.p, phiA_bar, sizeof(double) * M_, cudaMemcpyHostToDevice, st_));
@@ -328,7 +341,7 @@ void ModelAB::grad_w_sweep(const double* phiA_bar, const double* phiB_bar, doubl
     a.eF[0] = eFA_.p; a.eF[1] = eFB_.p;
     a.pA = pbA_.p; a.pB = pbB_.p;
     a.ds[0] = dsA_; a.ds[1] = dsB_;
-    a.chunk = reinterpret_cast<const Chunk*>(chunks_.p);
+    a.chunk = reinterpret_cast<const AdjointChunk*>(chunks_.p);
     a.partial = gpart_.p;
     a.M = M_;
     a.Ns = Ns_;
@@ -345,7 +358,7 @@ void ModelAB::stress_sweep(double* dFdl) {
     const int n[3] = {p_.Lx, p_.Ly, p_.Lz};
     const long st[3] = {(long)p_.Ly * p_.Lz, p_.Lz, 1};
     const double PI = 3.14159265358979323846;
-    if (sfrag_.n == 0) {
+    if (spart_.n == 0) {
         std::vector<double> f;
         for (int ax = 0; ax < 3; ax++) {
             sfo_[ax] = (int)f.size();

@@ -25,6 +25,19 @@ void DevBuf::alloc(size_t count) {
     n = count;
 }
 
+bool DevBuf::try_alloc(size_t count) {
+    release();
+    const cudaError_t e = cudaMalloc(&p, sizeof(double) * count);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();   // not an error of the caller's
+        p = nullptr;
+        return false;
+    }
+    PS_CUDA(e);
+    n = count;
+    return true;
+}
+
 void DevBuf::release() {
     if (p) cudaFree(p);
     p = nullptr;

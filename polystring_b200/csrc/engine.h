@@ -21,6 +21,7 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void alloc(size_t count);
+    bool try_alloc(size_t count);   // false where the device has no room
     void release();
     double2* c() const { return reinterpret_cast<double2*>(p); }
 };
@@ -148,6 +149,9 @@ private:
     bool batched_tables_ = false;
 };
 
+// steps t0 .. t1 - 1 of a chain, all in one block (adjoint_sweep.cu)
+struct AdjointChunk { int chain, blk, t0, t1; };
+
 // Model_AB on the device (Model_AB.cc:85-371 for a periodic cell)
 struct ModelABParams {
     int dim, Lx, Ly, Lz;
@@ -230,6 +234,7 @@ private:
     void ensure_adjoint_buffers(bool spec);
     // the adjoint on the persistent sweeps (adjoint_sweep.cu)
     bool sweep_adjoint(bool grad);
+    std::vector<AdjointChunk> adjoint_chunks() const;
     void forward_kept();
     void grad_w_sweep(const double* phiA_bar, const double* phiB_bar, double Q_bar, double* gA, double* gB);
     void stress_sweep(double* dFdl);
