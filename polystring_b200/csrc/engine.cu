@@ -759,21 +759,8 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
     cell_init(cell_);
     M_ = (long)Lx * Ly * Lz;
     PS_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    chain_ = new PairChain(Lx, Ly, Lz, scheme, 1);
-    if (scheme == SCHEME_OS2) {
-        chain_->set_tables(k_laplacian(cell_, Lx, Ly, Lz, ds), {});
-    } else if (scheme == SCHEME_ETDRK4) {
-        chain_->set_tables_etd(k2_orthogonal(cell_, Lx, Ly, Lz), ds, etd_M);
-    } else {
-        std::vector<double> k2 = k2_orthogonal(cell_, Lx, Ly, Lz);
-        std::vector<double> L1(M_), L2(M_);
-        for (long m = 0; m < M_; m++) {
-            L1[m] = exp(ds * k2[m]);
-            L2[m] = exp(0.5 * ds * k2[m]);
-        }
-        chain_->set_tables(L1, L2);
-    }
-    // one chain takes the persistent sweep as Model_AB's two do
+    // one chain takes the persistent sweep as Model_AB's two do; else the line passes,
+    // whose lane c carries zeros
     const char* force = getenv("PS_B200_LINE_PASSES");
     if (!(force && force[0] == '1') && (scheme == SCHEME_RQM4 || (scheme == SCHEME_OS2 && cell_separable(cell_))) &&
         RealSweep::supported(Lx, Ly, Lz)) {
@@ -781,12 +768,27 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
         double k[3];
         axis_k2(cell_, k);
         real_ = new RealSweep(n, k, ds, 1, scheme == SCHEME_OS2);
+    } else {
+        chain_ = new PairChain(Lx, Ly, Lz, scheme, 1);
+        if (scheme == SCHEME_OS2) {
+            chain_->set_tables(k_laplacian(cell_, Lx, Ly, Lz, ds), {});
+        } else if (scheme == SCHEME_ETDRK4) {
+            chain_->set_tables_etd(k2_orthogonal(cell_, Lx, Ly, Lz), ds, etd_M);
+        } else {
+            std::vector<double> k2 = k2_orthogonal(cell_, Lx, Ly, Lz);
+            std::vector<double> L1(M_), L2(M_);
+            for (long m = 0; m < M_; m++) {
+                L1[m] = exp(ds * k2[m]);
+                L2[m] = exp(0.5 * ds * k2[m]);
+            }
+            chain_->set_tables(L1, L2);
+        }
+        zero_.alloc(M_);
+        scratch_.alloc(M_);
+        launch_fill(zero_.p, M_, 0.0, st_);
     }
     eF_.alloc(2 * M_);
     eH_.alloc(2 * M_);
-    zero_.alloc(M_);
-    scratch_.alloc(M_);
-    launch_fill(zero_.p, M_, 0.0, st_);
     PS_CUDA(cudaStreamSynchronize(st_));
 }
 

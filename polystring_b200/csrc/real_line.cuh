@@ -148,7 +148,11 @@ struct RealKernel {
         for (int m = 0; m < N; m++) cosn[m] = cosl(2.0L * pi * m / N);
         for (int d = 0; d < N; d++) {
             long double a = 0.0L;
-            for (int k = 0; k < N; k++) a += (long double)L[k] * cosn[(int)((long)k * d % N)];
+            for (int k = 0, kd = 0; k < N; k++) {   // kd = k d mod N
+                a += (long double)L[k] * cosn[kd];
+                kd += d;
+                if (kd >= N) kd -= N;
+            }
             c[d] = a / N;
         }
         for (int h = 0; h < 2; h++)
