@@ -435,7 +435,7 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
         throw Error(-4, "contour quadrature precondition fails for Ms = [" + std::to_string(p.sA) + ", " +
                             std::to_string(p.sB) + "]");
     PS_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    chain_ = new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : p.mde == 2 ? SCHEME_ETDRK4 : SCHEME_RQM4, 1);
+    chain_.reset(new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : p.mde == 2 ? SCHEME_ETDRK4 : SCHEME_RQM4, 1));
     // k tables.  ds of the two blocks agree to within two ulps (both round
     // 1/(LA+LB)); the packed lanes share the block-A table.
     if (p.mde == 1) {
@@ -461,7 +461,7 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
         const int n[3] = {p.Lx, p.Ly, p.Lz};
         double k[3];
         axis_k2(p_.cell, k);
-        real_ = new RealSweep(n, k, dsA_, 2, p.mde == 1);
+        real_.reset(new RealSweep(n, k, dsA_, 2, p.mde == 1));
     }
     hf_.alloc((size_t)(Ns_ + 1) * M_);
     hc_.alloc((size_t)(Ns_ + 1) * M_);
@@ -499,8 +499,6 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
 ModelAB::~ModelAB() {
     if (gprop_) cudaGraphExecDestroy(gprop_);
     if (gpost_) cudaGraphExecDestroy(gpost_);
-    delete chain_;
-    delete real_;
     if (axs_) cudaFree(axs_);
     if (st_) cudaStreamDestroy(st_);
 }
@@ -767,9 +765,9 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
         const int n[3] = {Lx, Ly, Lz};
         double k[3];
         axis_k2(cell_, k);
-        real_ = new RealSweep(n, k, ds, 1, scheme == SCHEME_OS2);
+        real_.reset(new RealSweep(n, k, ds, 1, scheme == SCHEME_OS2));
     } else {
-        chain_ = new PairChain(Lx, Ly, Lz, scheme, 1);
+        chain_.reset(new PairChain(Lx, Ly, Lz, scheme, 1));
         if (scheme == SCHEME_OS2) {
             chain_->set_tables(k_laplacian(cell_, Lx, Ly, Lz, ds), {});
         } else if (scheme == SCHEME_ETDRK4) {
@@ -793,8 +791,6 @@ UpdaterCtx::UpdaterCtx(int scheme, const Cell& cell, int Lx, int Ly, int Lz, dou
 }
 
 UpdaterCtx::~UpdaterCtx() {
-    delete chain_;
-    delete real_;
     if (st_) cudaStreamDestroy(st_);
 }
 

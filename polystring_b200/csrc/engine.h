@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <memory>
 #include <vector>
 
 #include "ps_internal.h"
@@ -194,7 +195,7 @@ public:
     void check() const { if (real_) real_->check(); }
     const ModelABParams& params() const { return p_; }
     bool persistent_sweep() const { return real_ != nullptr; }
-    const RealSweep* sweep() const { return real_; }
+    const RealSweep* sweep() const { return real_.get(); }
     // the sweep's description of this solve (its own work fields, barrier
     // words and error flag)
     RealProblem sweep_descriptor() const;
@@ -213,7 +214,7 @@ public:
     void stress_checkpointed(int k, double* dFdl);
     // for BatchAB: the chain histories and factors, the post-propagator work
     // (Q, densities, field update) on a given stream, and the iteration count
-    PairChain* chain() const { return chain_; }
+    PairChain* chain() const { return chain_.get(); }
     double* hist_f() const { return hf_.p; }
     double* hist_c() const { return hc_.p; }
     const double* factor(int full, int block) const {
@@ -244,8 +245,8 @@ private:
     int LA_, LB_, Ns_;
     double dsA_, dsB_;
     int ruleA_, ruleB_;
-    PairChain* chain_ = nullptr;
-    RealSweep* real_ = nullptr;          // persistent sweep (3D grids, RQM4 and OS2)
+    std::unique_ptr<PairChain> chain_;
+    std::unique_ptr<RealSweep> real_;    // persistent sweep (RQM4 and OS2, where the grid has one)
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t gprop_ = nullptr, gpost_ = nullptr;
     DevBuf hf_, hc_, wA_, wB_, yita_, phiA_, phiB_, eFA_, eHA_, eFB_, eHB_;
@@ -303,7 +304,7 @@ public:
     void count_iterations(int n) { iter_ += n; }
     bool has_fields() const { return fields_set_; }
     // for batches (batch_ab.cu): the packed chain, histories and factors
-    PairChain* chain() const { return chain_; }
+    PairChain* chain() const { return chain_.get(); }
     double* hist_f() const { return hf_.p; }
     double* hist_c() const { return hc_.p; }
     const double* factor(int full, int block) const { return full ? eF_[block].p : eH_[block].p; }
@@ -312,7 +313,7 @@ public:
     int launches_post() const { return mean_launches(M_) + density_launches(M_, 3) + (p_.scft == 1 ? 4 : 1); }
     // the persistent sweep with three factor sets
     bool persistent_sweep() const { return real_ != nullptr; }
-    const RealSweep* sweep() const { return real_; }
+    const RealSweep* sweep() const { return real_.get(); }
     RealProblem sweep_descriptor() const;
     const ModelABCParams& params() const { return p_; }
 
@@ -322,7 +323,7 @@ private:
     long M_;
     int L_[3], Ns_;
     double ds_[3];
-    PairChain* chain_ = nullptr;
+    std::unique_ptr<PairChain> chain_;
     cudaStream_t st_ = nullptr;
     DevBuf hf_, hc_, w_[3], yita_, phi_[3], eF_[3], eH_[3], c_[3], scal_, partial_;
     DevBuf hw_[3], hd_[3], B_[3];
@@ -330,7 +331,7 @@ private:
     cudaGraphExec_t graph_ = nullptr;
     long iter_ = 0;
     bool fields_set_ = false;
-    RealSweep* real_ = nullptr;
+    std::unique_ptr<RealSweep> real_;
 };
 
 // Single propagator updater behind the Updater C-ABI (RQM4 / OS2 / ETDRK4)
@@ -351,8 +352,8 @@ private:
     double ds_;
     int etd_M_;
     long M_;
-    PairChain* chain_ = nullptr;
-    RealSweep* real_ = nullptr;
+    std::unique_ptr<PairChain> chain_;
+    std::unique_ptr<RealSweep> real_;
     DevBuf eF_, eH_, zero_, scratch_, dw_, dqs_;
     cudaStream_t st_ = nullptr;
 };

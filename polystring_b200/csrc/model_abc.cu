@@ -54,7 +54,7 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
                                 std::to_string(p.s[x]) + ")");
     }
     PS_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    chain_ = new PairChain(p.Lx, p.Ly, p.Lz, SCHEME_RQM4, 1);
+    chain_.reset(new PairChain(p.Lx, p.Ly, p.Lz, SCHEME_RQM4, 1));
     // the packed lanes share the block-A tables; the three ds agree to a
     // few ulps (each rounds 1 / L)
     std::vector<double> k2 = k2_orthogonal(p_.cell, p.Lx, p.Ly, p.Lz);
@@ -69,7 +69,7 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
         const int n[3] = {p.Lx, p.Ly, p.Lz};
         double k[3];
         axis_k2(p_.cell, k);
-        real_ = new RealSweep(n, k, ds_[0], 2, false);
+        real_.reset(new RealSweep(n, k, ds_[0], 2, false));
     }
     hf_.alloc((size_t)(Ns_ + 1) * M_);
     hc_.alloc((size_t)(Ns_ + 1) * M_);
@@ -97,8 +97,6 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
 
 ModelABC::~ModelABC() {
     if (graph_) cudaGraphExecDestroy(graph_);
-    delete chain_;
-    delete real_;
     if (axs_) cudaFree(axs_);
     if (st_) cudaStreamDestroy(st_);
 }

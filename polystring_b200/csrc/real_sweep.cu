@@ -563,6 +563,15 @@ bool RealSweep::supported(int Lx, int Ly, int Lz) {
 }
 
 RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool os2) : nl_(nl), os2_(os2) {
+    try {
+        init(n, k, ds, nl, os2);
+    } catch (...) {
+        release();
+        throw;
+    }
+}
+
+void RealSweep::init(const int n[3], const double k[3], double ds, int nl, bool os2) {
     std::copy(n, n + 3, n_);
     dim_ = n[2] > 1 ? 3 : n[1] > 1 ? 2 : 1;
     const size_t M = (size_t)n[0] * n[1] * n[2];
@@ -591,14 +600,14 @@ RealSweep::RealSweep(const int n[3], const double k[3], double ds, int nl, bool 
     PS_CUDA(cudaMemcpy(frag_, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
     PS_CUDA(cudaMalloc(&bar_, 33 * sizeof(unsigned)));
     PS_CUDA(cudaMemset(bar_, 0, 33 * sizeof(unsigned)));
-    if (dim_ == 3 || (tile_ && !cluster_)) {
-        notice_ = notices().take();
-    }
+    if (dim_ == 3 || (tile_ && !cluster_)) notice_ = notices().take();
     const char* polls = getenv("PS_B200_BARRIER_POLLS");
     polls_ = polls ? std::max(0, atoi(polls)) : kBarrierPolls;
 }
 
-RealSweep::~RealSweep() {
+RealSweep::~RealSweep() { release(); }
+
+void RealSweep::release() {
     cudaFree(work_);
     cudaFree(frag_);
     cudaFree(bar_);

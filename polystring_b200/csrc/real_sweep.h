@@ -131,6 +131,8 @@ public:
     void reset(cudaStream_t st);
 
 private:
+    void init(const int n[3], const double k[3], double ds, int nl, bool os2);
+    void release();
     int n_[3], dim_, nl_, os2_, ncta_, variant_, fo_[3], nfrag_;
     bool tile_ = false;
     int cluster_ = 0;   // CTAs of a chain's cluster (0: chains over the grid)

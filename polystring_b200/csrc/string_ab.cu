@@ -192,7 +192,7 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
         throw Error(-4, "contour quadrature precondition fails");
     if (p.mde != 0 && p.mde != 1) throw Error(-2, "string images use RQM4 or OS2");
     PS_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    chain_ = new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : SCHEME_RQM4, nloc_);
+    chain_.reset(new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : SCHEME_RQM4, nloc_));
     // every image's chains in one launch of a persistent sweep per SCFT iteration
     // where the 2D grid has one (PS_B200_LINE_PASSES=1 keeps the batched line
     // passes)
@@ -204,7 +204,7 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
         const int n[3] = {p.Lx, p.Ly, 1};
         double k[3];
         axis_k2(p_.cell, k);
-        real_ = new RealSweep(n, k, dsA_, 2, p.mde == 1);
+        real_.reset(new RealSweep(n, k, dsA_, 2, p.mde == 1));
     }
     if (p.mde == 1) {
         chain_->set_tables(k_laplacian(p_.cell, p.Lx, p.Ly, p.Lz, dsA_), {});
@@ -279,8 +279,6 @@ StringAB::~StringAB() {
     if (giter_) cudaGraphExecDestroy(giter_);
     if (grelax_) cudaGraphExecDestroy(grelax_);
     if (grepar_) cudaGraphExecDestroy(grepar_);
-    delete chain_;
-    delete real_;
     cudaFree(images_);
     if (st_) cudaStreamDestroy(st_);
 }

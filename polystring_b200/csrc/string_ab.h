@@ -45,11 +45,11 @@ private:
     long M_;
     int LA_, LB_, Ns_;
     double dsA_, dsB_;
-    PairChain* chain_ = nullptr;
+    std::unique_ptr<PairChain> chain_;
     cudaStream_t st_ = nullptr;
     cudaGraphExec_t giter_ = nullptr, grelax_ = nullptr, grepar_ = nullptr;
     DevBuf hf_, hc_, wa_, wb_, yita_, phiA_, phiB_, eFA_, eHA_, eFB_, eHB_, ends_, cA_, cB_, scal_, S_, partial_;
-    RealSweep* real_ = nullptr;          // operators of the images' persistent sweeps
+    std::unique_ptr<RealSweep> real_;    // operators of the images' persistent sweeps
     RealProblem* images_ = nullptr;      // the images' descriptions on the device
     bool tiled_ = false;                 // an axis past 64 points: a cluster an image (tile_sweep.cu),
                                          // else a CTA a chain (plane_sweep.cu)
