@@ -146,14 +146,15 @@ struct RealKernel {
         const long double pi = 3.141592653589793238462643383279502884L;
         std::vector<long double> cosn(N), c(N);
         for (int m = 0; m < N; m++) cosn[m] = cosl(2.0L * pi * m / N);
-        for (int d = 0; d < N; d++) {
+        // even in d, and its terms in k
+        for (int d = 0; d <= N / 2; d++) {
             long double a = 0.0L;
-            for (int k = 0, kd = 0; k < N; k++) {   // kd = k d mod N
-                a += (long double)L[k] * cosn[kd];
+            for (int k = 1, kd = d; k < N / 2; k++) {   // kd = k d mod N
+                a += L[k] * cosn[kd];
                 kd += d;
                 if (kd >= N) kd -= N;
             }
-            c[d] = a / N;
+            c[d] = c[(N - d) % N] = (2.0L * a + L[0] + (d & 1 ? -L[N / 2] : L[N / 2])) / N;
         }
         for (int h = 0; h < 2; h++)
             for (int d = 0; d < N; d++) half[h].push_back(h ? c[d] - c[(d + N / 2) % N] : c[d] + c[(d + N / 2) % N]);
