@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(k1T, 1) line_sweep_kernel(const __grid_constan
         v[2] = vp + vm;
         v[3] = vp - vm;
     };
-    double q[4] = {0.0, 0.0, 0.0, 0.0}, e[4] = {0.0, 0.0, 0.0, 0.0}, w[4], z[4];
+    double q[4] = {0.0, 0.0, 0.0, 0.0}, e[4] = {0.0, 0.0, 0.0, 0.0}, f[4] = {0.0, 0.0, 0.0, 0.0}, w[4], z[4];
     if (own)
 #pragma unroll
         for (int i = 0; i < 4; i++) q[i] = __ldg(L.hist + R::point(i, o));
@@ -343,11 +343,14 @@ __global__ void __launch_bounds__(k1T, 1) line_sweep_kernel(const __grid_constan
             const int b = lane_block(L, t);
             if (t == 0 || b != lane_block(L, t - 1))
 #pragma unroll
-                for (int i = 0; i < 4; i++) e[i] = __ldg((p.os2 ? L.eF[b] : L.eH[b]) + R::point(i, o));
+                for (int i = 0; i < 4; i++) {
+                    f[i] = __ldg(L.eF[b] + R::point(i, o));
+                    e[i] = __ldg(L.eH[b] + R::point(i, o));
+                }
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 z[i] = __dmul_rn(q[i], e[i]);
-                w[i] = p.os2 ? z[i] : __dmul_rn(z[i], e[i]);
+                w[i] = __dmul_rn(q[i], f[i]);
             }
             put(0, w[0], w[1], w[2], w[3]);
             if (!p.os2) put(1, z[0], z[1], z[2], z[3]);
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(k1T, 1) line_sweep_kernel(const __grid_constan
             if (own) {
                 take(1, z);
 #pragma unroll
-                for (int i = 0; i < 4; i++) z[i] = __dmul_rn(z[i], __dmul_rn(e[i], e[i]));
+                for (int i = 0; i < 4; i++) z[i] = __dmul_rn(z[i], f[i]);
                 put(1, z[0], z[1], z[2], z[3]);
             }
             __syncthreads();
@@ -377,9 +380,8 @@ __global__ void __launch_bounds__(k1T, 1) line_sweep_kernel(const __grid_constan
             double* out = L.hist + (long)(t + 1) * N;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                q[i] = p.os2 ? __dmul_rn(w[i], e[i])
-                             : div_rn(fma(4.0, __dmul_rn(z[i], e[i]), -__dmul_rn(w[i], __dmul_rn(e[i], e[i]))), 3.0,
-                                      1.0 / 3.0);
+                w[i] = __dmul_rn(w[i], f[i]);
+                q[i] = p.os2 ? w[i] : div_rn(fma(4.0, __dmul_rn(z[i], e[i]), -w[i]), 3.0, 1.0 / 3.0);
                 out[R::point(i, o)] = q[i];
             }
         }
