@@ -128,7 +128,7 @@ public:
     // kernel launches per pair step
     int launches_per_step() const;
     // ETDRK4: whether all steps run in one launch
-    bool small_etd() const;
+    bool small_etd() const { return small_etd_; }
     long M() const { return M_; }
     const AxisPlan& plan() const { return plan_; }
     // work fields and tables (for grouped launches over many chains)
@@ -147,7 +147,7 @@ private:
     AxisPlan plan_;
     DevBuf z_[3], u_[2], L1_, L2_, half_;
     DevBuf etd_, etdtab_;   // ETDRK4: V, Nv, A, Na, Nb (packed spectra); E, E2, Q, f1, f2, f3
-    bool batched_tables_ = false;
+    bool batched_tables_ = false, small_etd_ = false;
 };
 
 // steps t0 .. t1 - 1 of a chain, all in one block (adjoint_sweep.cu)

@@ -462,7 +462,10 @@ void PairChain::set_tables_etd(const std::vector<double>& k2, double ds, int Mc)
         tab[4 * M + m] = ds * (s2 / Mc);
         tab[5 * M + m] = ds * (s3 / Mc);
     }
-    if (small_etd()) {
+    // PS_B200_LINE_PASSES=1 at this point keeps the line passes
+    const char* force = getenv("PS_B200_LINE_PASSES");
+    small_etd_ = small_grid(Lx_, Ly_, Lz_) && !(force && force[0] == '1');
+    if (small_etd_) {
         small_kernel(M_, [](auto kernel, int) {
             PS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         });
@@ -475,12 +478,6 @@ void PairChain::set_tables_etd(const std::vector<double>& k2, double ds, int Mc)
     }
     etdtab_.alloc(tab.size());
     PS_CUDA(cudaMemcpy(etdtab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
-}
-
-// PS_B200_LINE_PASSES=1 keeps the line passes
-bool PairChain::small_etd() const {
-    const char* force = getenv("PS_B200_LINE_PASSES");
-    return scheme_ == SCHEME_ETDRK4 && small_grid(Lx_, Ly_, Lz_) && !(force && force[0] == '1');
 }
 
 // forward (MODE_FWD) or inverse (MODE_INV, unnormalised) transform of one
@@ -508,7 +505,7 @@ void PairChain::enqueue_etd(double* hf, double* hc, int nsteps, const LaneFactor
     f.T = T;
     f.V = etd_.c(); f.Nv = f.V + M; f.A = f.V + 2 * M; f.Na = f.V + 3 * M; f.Nb = f.V + 4 * M;
     f.E = etdtab_.p; f.E2 = f.E + M; f.Q = f.E + 2 * M; f.f1 = f.E + 3 * M; f.f2 = f.E + 4 * M; f.f3 = f.E + 5 * M;
-    if (small_etd()) {
+    if (small_etd_) {
         EtdSmall a{};
         a.hf = hf;
         a.hc = c_in_fixed ? nullptr : hc;   // a fixed lane c is zero (UpdaterCtx)
