@@ -300,9 +300,9 @@ void ModelAB::grad_w_sweep(const double* phiA_bar, const double* phiB_bar, doubl
         w.insert(w.end(), wAf.begin(), wAf.end());
         w.insert(w.end(), wBf.begin(), wBf.end());
         srcw_.alloc(w.size());
-        PS_CUDA(cudaMemcpy(srcw_.p, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice));
+        upload(srcw_.p, w.data(), sizeof(double) * w.size());
         chunks_.alloc((sizeof(AdjointChunk) * ch.size() + 7) / 8);
-        PS_CUDA(cudaMemcpy(chunks_.p, ch.data(), sizeof(AdjointChunk) * ch.size(), cudaMemcpyHostToDevice));
+        upload(chunks_.p, ch.data(), sizeof(AdjointChunk) * ch.size());
         adj_chunks_ = (int)ch.size();
     }
     PS_CUDA(cudaMemcpyAsync(pbA_.p, phiA_bar, sizeof(double) * M_, cudaMemcpyHostToDevice, st_));
@@ -371,7 +371,7 @@ void ModelAB::stress_sweep(double* dFdl) {
             real_fragments(n[ax], r2, f);
         }
         sfrag_.alloc(f.size());
-        PS_CUDA(cudaMemcpy(sfrag_.p, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
+        upload(sfrag_.p, f.data(), sizeof(double) * f.size());
         spart_.alloc(3 * kStressCtas);
     }
     forward_kept();

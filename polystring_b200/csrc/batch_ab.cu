@@ -153,7 +153,7 @@ void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per,
         }
     }
     PS_CUDA(cudaMalloc(&c.dev, sizeof(RealProblem) * d.size()));
-    PS_CUDA(cudaMemcpy(c.dev, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+    upload(c.dev, d.data(), sizeof(RealProblem) * d.size());
 }
 
 void BatchAB::build_sweeps(const std::vector<int>& members) {
@@ -297,7 +297,7 @@ void BatchAB::build_group(Group& g) {
         g.Ns_max = std::max(g.Ns_max, d[i].Ns);
     }
     PS_CUDA(cudaMalloc(&g.dev, sizeof(GroupSolve) * d.size()));
-    PS_CUDA(cudaMemcpy(g.dev, d.data(), sizeof(GroupSolve) * d.size(), cudaMemcpyHostToDevice));
+    upload(g.dev, d.data(), sizeof(GroupSolve) * d.size());
     for (int k = 0; k < 9; k++) {
         const int mode = kPass[k][0], ax = kPass[k][1], p3 = kPass[k][2];
         if (ax == GROUP_AX_MID && g.naxes < 3) continue;
@@ -310,7 +310,7 @@ void BatchAB::build_group(Group& g) {
         }
         if (g.smem[k] > kLinePassSmemLimit) throw Error(-2, "a batched line pass tile does not fit in shared memory");
         PS_CUDA(cudaMalloc(&g.prefix_dev[k], sizeof(int) * pre.size()));
-        PS_CUDA(cudaMemcpy(g.prefix_dev[k], pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice));
+        upload(g.prefix_dev[k], pre.data(), sizeof(int) * pre.size());
     }
 }
 

@@ -262,20 +262,20 @@ PairChain::PairChain(int Lx, int Ly, int Lz, int scheme, int nbatch)
 
 void PairChain::set_tables(const std::vector<double>& L1, const std::vector<double>& L2) {
     L1_.alloc(M_);
-    PS_CUDA(cudaMemcpy(L1_.p, L1.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
+    upload(L1_.p, L1.data(), sizeof(double) * M_);
     if (scheme_ == SCHEME_RQM4) {
         L2_.alloc(M_);
-        PS_CUDA(cudaMemcpy(L2_.p, L2.data(), sizeof(double) * M_, cudaMemcpyHostToDevice));
+        upload(L2_.p, L2.data(), sizeof(double) * M_);
     }
     batched_tables_ = false;
 }
 
 void PairChain::set_tables_batched(const std::vector<double>& L1, const std::vector<double>& L2) {
     L1_.alloc((size_t)M_ * nbatch_);
-    PS_CUDA(cudaMemcpy(L1_.p, L1.data(), sizeof(double) * M_ * nbatch_, cudaMemcpyHostToDevice));
+    upload(L1_.p, L1.data(), sizeof(double) * M_ * nbatch_);
     if (scheme_ == SCHEME_RQM4) {
         L2_.alloc((size_t)M_ * nbatch_);
-        PS_CUDA(cudaMemcpy(L2_.p, L2.data(), sizeof(double) * M_ * nbatch_, cudaMemcpyHostToDevice));
+        upload(L2_.p, L2.data(), sizeof(double) * M_ * nbatch_);
     }
     batched_tables_ = true;
 }
@@ -469,8 +469,8 @@ ModelAB::ModelAB(const ModelABParams& p, bool batch_member) : p_(p) {
     phiA_.alloc(M_); phiB_.alloc(M_);
     eFA_.alloc(M_); eHA_.alloc(M_); eFB_.alloc(M_); eHB_.alloc(M_);
     cA_.alloc(cA.size()); cB_.alloc(cB.size());
-    PS_CUDA(cudaMemcpy(cA_.p, cA.data(), sizeof(double) * cA.size(), cudaMemcpyHostToDevice));
-    PS_CUDA(cudaMemcpy(cB_.p, cB.data(), sizeof(double) * cB.size(), cudaMemcpyHostToDevice));
+    upload(cA_.p, cA.data(), sizeof(double) * cA.size());
+    upload(cB_.p, cB.data(), sizeof(double) * cB.size());
     scal_.alloc(32);
     partial_.alloc((size_t)kRedBlocks * 64);
     if (p.scft == 1) {

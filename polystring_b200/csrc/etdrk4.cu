@@ -477,7 +477,7 @@ void PairChain::set_tables_etd(const std::vector<double>& k2, double ds, int Mc)
         etd_pass<ETD_INV>(plan_.ax[a], nullptr, nullptr);
     }
     etdtab_.alloc(tab.size());
-    PS_CUDA(cudaMemcpy(etdtab_.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+    upload(etdtab_.p, tab.data(), sizeof(double) * tab.size());
 }
 
 // forward (MODE_FWD) or inverse (MODE_INV, unnormalised) transform of one

@@ -77,7 +77,7 @@ ModelABC::ModelABC(const ModelABCParams& p) : p_(p) {
     for (int x = 0; x < 3; x++) {
         w_[x].alloc(M_); phi_[x].alloc(M_); eF_[x].alloc(M_); eH_[x].alloc(M_);
         c_[x].alloc(cw[x].size());
-        PS_CUDA(cudaMemcpy(c_[x].p, cw[x].data(), sizeof(double) * cw[x].size(), cudaMemcpyHostToDevice));
+        upload(c_[x].p, cw[x].data(), sizeof(double) * cw[x].size());
     }
     scal_.alloc(32);
     partial_.alloc((size_t)kRedBlocks * 128);

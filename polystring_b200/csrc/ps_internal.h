@@ -25,6 +25,14 @@ void set_last_error(const std::string& msg);
             throw ::ps::Error(-3, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Copies tables to the device, and waits until they are there: cudaMemcpy may return
+// when a small copy from pageable memory is only staged, and the contexts' streams do not
+// wait for the stream it is staged in.
+inline void upload(void* dst, const void* src, size_t bytes) {
+    PS_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    PS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // ---------------------------------------------------------------------------
 // line passes (kernels in line_pass.cu)
 // ---------------------------------------------------------------------------

@@ -597,9 +597,10 @@ void RealSweep::init(const int n[3], const double k[3], double ds, int nl, bool 
         PS_CUDA(cudaMalloc(&work_, sizeof(double) * 2 * nl * M));
     }
     PS_CUDA(cudaMalloc(&frag_, sizeof(double) * f.size()));
-    PS_CUDA(cudaMemcpy(frag_, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice));
+    upload(frag_, f.data(), sizeof(double) * f.size());
     PS_CUDA(cudaMalloc(&bar_, 33 * sizeof(unsigned)));
-    PS_CUDA(cudaMemset(bar_, 0, 33 * sizeof(unsigned)));
+    const unsigned zeros[33] = {};
+    upload(bar_, zeros, sizeof(zeros));
     if (dim_ == 3 || (tile_ && !cluster_)) notice_ = notices().take();
     const char* polls = getenv("PS_B200_BARRIER_POLLS");
     polls_ = polls ? std::max(0, atoi(polls)) : kBarrierPolls;

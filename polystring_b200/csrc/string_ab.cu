@@ -230,7 +230,7 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
                 for (int y = 0; y < p.Ly; y++) kt.push_back(exp(h * k2[(long)y * p.Lz]));
             }
             clK_.alloc(kt.size());
-            PS_CUDA(cudaMemcpy(clK_.p, kt.data(), sizeof(double) * kt.size(), cudaMemcpyHostToDevice));
+            upload(clK_.p, kt.data(), sizeof(double) * kt.size());
         }
     }
     if (!use_cluster_ && !real_) chain_->autotune(st_);
@@ -256,11 +256,11 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
         }
         if (tiled_) tile_string_prepare(d[0], nloc_);
         PS_CUDA(cudaMalloc(&images_, sizeof(RealProblem) * d.size()));
-        PS_CUDA(cudaMemcpy(images_, d.data(), sizeof(RealProblem) * d.size(), cudaMemcpyHostToDevice));
+        upload(images_, d.data(), sizeof(RealProblem) * d.size());
     }
     cA_.alloc(cA.size()); cB_.alloc(cB.size());
-    PS_CUDA(cudaMemcpy(cA_.p, cA.data(), sizeof(double) * cA.size(), cudaMemcpyHostToDevice));
-    PS_CUDA(cudaMemcpy(cB_.p, cB.data(), sizeof(double) * cB.size(), cudaMemcpyHostToDevice));
+    upload(cA_.p, cA.data(), sizeof(double) * cA.size());
+    upload(cB_.p, cB.data(), sizeof(double) * cB.size());
     scal_.alloc((size_t)8 * m);
     S_.alloc(m);
     partial_.alloc((size_t)kBG * m * 8);

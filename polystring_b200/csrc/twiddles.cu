@@ -33,7 +33,7 @@ const double2* twiddle_table(int N) {
     }
     double2* d = nullptr;
     PS_CUDA(cudaMalloc(&d, sizeof(double2) * N));
-    PS_CUDA(cudaMemcpy(d, h.data(), sizeof(double2) * N, cudaMemcpyHostToDevice));
+    upload(d, h.data(), sizeof(double2) * N);
     g_tw[key] = d;
     return d;
 }
