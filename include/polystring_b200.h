@@ -22,7 +22,7 @@
  *
  * A sweep over many CTAs that are kept from running together (by another program's
  * kernels, say) gives up at its grid barrier after some ten seconds
- * (PS_B200_BARRIER_POLLS=n: after n polls).  The model's and batch's calls that wait
+ * (PS_B200_BARRIER_GIVE_UP=1: at once, for tests).  The model's and batch's calls that wait
  * for results, and the next iteration, then return PS_ERR_CUDA until fields are set
  * again; an updater's see ps_updater_check.
  *

@@ -145,6 +145,7 @@ void BatchAB::add_chunk(const std::vector<int>& ks, const std::vector<int>& per,
         PS_CUDA(cudaMalloc(&c.bar, 32 * sizeof(unsigned) * d.size()));
         for (int i = 0; i < c.n; i++) {
             d[i].bar = c.bar + 32 * (size_t)i;
+            c.hasty = d[i].hasty;
             d[i].cta0 = c.grid;
             d[i].ncta = per[i];
             c.grid += 2 * per[i];
@@ -323,7 +324,7 @@ void BatchAB::enqueue_iteration() {
             tile_cluster_launch_many(c.dev, c.n, c.cluster, c.smem, st_);
         } else {
             PS_CUDA(cudaMemsetAsync(c.bar, 0, 32 * sizeof(unsigned) * (size_t)c.n, st_));
-            real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, st_);
+            real_sweep_launch_many(c.dev, c.n, c.smem, c.wide, c.grid, c.hasty, st_);
         }
         launches++;
     }

@@ -43,7 +43,7 @@ private:
     // solves that share a sweep launch: their descriptors on the device, and
     // 32 barrier words each (3D)
     struct SweepChunk {
-        int n = 0, grid = 0, pairs = 0;
+        int n = 0, grid = 0, pairs = 0, hasty = 0;
         int cluster = 0;
         bool plane = false, wide = false;
         size_t smem = 0;

@@ -531,7 +531,7 @@ void ModelAB::set_fields(const double* wA, const double* wB, bool dev) {
     if (p_.scft == 1) init_anderson(wA, wB, dev);
     launch_factors(wA_.p, wB_.p, M_, dsA_, dsB_, eFA_.p, eHA_.p, eFB_.p, eHB_.p, 1, 0, st_);
     PS_CUDA(cudaStreamSynchronize(st_));
-    if (real_) real_->reset(st_);
+    if (real_) real_->reset();
     iter_ = 0;
     fields_set_ = true;
     forward_done_ = false;
@@ -837,7 +837,7 @@ void UpdaterCtx::solve_host(const double* w, double* qs, int len) {
 
 void UpdaterCtx::check() {
     if (!real_ || !real_->failed()) return;
-    real_->reset(st_);
+    real_->reset();
     throw Error(-3, "a propagator sweep gave up at a grid barrier (its CTAs were not all running)");
 }
 

@@ -125,7 +125,7 @@ void ModelABC::set_fields(const double* const w[3], bool dev) {
     launch_factors(w_[0].p, w_[1].p, M_, ds_[0], ds_[1], eF_[0].p, eH_[0].p, eF_[1].p, eH_[1].p, 1, 0, st_);
     launch_factors(w_[2].p, w_[2].p, M_, ds_[2], ds_[2], eF_[2].p, eH_[2].p, eF_[2].p, eH_[2].p, 1, 0, st_);
     PS_CUDA(cudaStreamSynchronize(st_));
-    if (real_) real_->reset(st_);
+    if (real_) real_->reset();
     iter_ = 0;
     fields_set_ = true;
 }

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kNT, ONE ? 1 : 2) real_sweep_kernel(const __gr
         if (t >= 0) {
             run_x<ONE>(p, frx, xcache, ch, t, w, nw);
             target += ncta;
-            if (!chain_barrier(p, bar, target)) return;
+            if (!chain_barrier(bar, p.err, &p.notice, one.hasty, target)) return;
         }
         for (int slab = cta; slab < p.Lx; slab += ncta) {
             if (t >= 0) {
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kNT, ONE ? 1 : 2) real_sweep_kernel(const __gr
         }
         if (t + 1 < p.Ns) {
             target += ncta;
-            if (!chain_barrier(p, bar, target)) return;
+            if (!chain_barrier(bar, p.err, &p.notice, one.hasty, target)) return;
         }
     }
 }
@@ -516,8 +516,10 @@ void real_sweep_launch(const RealProblem& p0, int ncta, cudaStream_t st) {
     launch(p, nullptr, 0, smem, true, ncta * p.nl, st);
 }
 
-void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool one, int grid, cudaStream_t st) {
-    launch(RealProblem{}, d, n, smem, one, grid, st);
+void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool one, int grid, int hasty, cudaStream_t st) {
+    RealProblem all{};
+    all.hasty = hasty;
+    launch(all, d, n, smem, one, grid, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -602,8 +604,8 @@ void RealSweep::init(const int n[3], const double k[3], double ds, int nl, bool 
     const unsigned zeros[33] = {};
     upload(bar_, zeros, sizeof(zeros));
     if (dim_ == 3 || (tile_ && !cluster_)) notice_ = notices().take();
-    const char* polls = getenv("PS_B200_BARRIER_POLLS");
-    polls_ = polls ? std::max(0, atoi(polls)) : kBarrierPolls;
+    const char* hasty = getenv("PS_B200_BARRIER_GIVE_UP");
+    hasty_ = hasty && hasty[0] == '1';
 }
 
 RealSweep::~RealSweep() { release(); }
@@ -627,7 +629,7 @@ RealProblem RealSweep::problem(const RealLane* lanes, int Ns) const {
     p.bar = bar_;
     p.err = reinterpret_cast<int*>(bar_ + 32);
     p.notice = notice_;
-    p.polls = polls_;
+    p.hasty = hasty_;
     p.Lx = n_[0]; p.Ly = n_[1]; p.Lz = n_[2];
     p.Ns = Ns;
     p.nl = nl_;
@@ -640,7 +642,7 @@ void RealSweep::enqueue(const RealProblem& p, cudaStream_t st) const {
     if (dim_ == 1) return line_sweep_launch(p, st);
     if (dim_ == 2 && !tile_) return plane_sweep_launch(p, st);
     if (cluster_) return tile_cluster_launch(p, cluster_, st);
-    PS_CUDA(cudaMemsetAsync(bar_, 0, 33 * sizeof(unsigned), st));
+    PS_CUDA(cudaMemsetAsync(bar_, 0, 32 * sizeof(unsigned), st));
     if (tile_) return tile_sweep_launch(p, ncta_, st);
     real_sweep_launch(p, ncta_, st);
 }
@@ -651,9 +653,11 @@ void RealSweep::check() const {
     if (failed()) throw Error(-3, "a propagator sweep gave up at a grid barrier (its CTAs were not all running)");
 }
 
-void RealSweep::reset(cudaStream_t st) {
+void RealSweep::reset() {
     if (!failed()) return;
-    PS_CUDA(cudaMemsetAsync(bar_ + 32, 0, sizeof(unsigned), st));
+    PS_CUDA(cudaDeviceSynchronize());   // a sweep still queued stops at the flag without a notice of its own
+    const unsigned zero = 0;
+    upload(bar_ + 32, &zero, sizeof(zero));
     *((volatile int*)notice_) = 0;
 }
 

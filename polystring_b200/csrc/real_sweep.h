@@ -35,7 +35,7 @@ struct RealProblem {
     unsigned* bar;        // barrier counters (one a chain, 16 words apart), zeroed before the launch
     int* err;             // nonzero after a barrier timeout, for the chains' CTAs
     int* notice;          // the same in host memory
-    int polls;            // after which a barrier gives up
+    int hasty;            // barriers give up at the first poll in vain (of a launch: its `one`'s)
     int Lx, Ly, Lz, Ns, nl;
     int os2;              // second-order splitting: full steps only
     int xcols;            // columns of an x-pass task (a multiple of 8)
@@ -66,7 +66,7 @@ int real_sweep_columns(int variant);
 void real_sweep_launch(const RealProblem& p, int ncta, cudaStream_t st);
 // n solves described in device memory (shapes may differ), grid CTAs in all, the
 // largest of the solves' shared memory
-void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool wide, int grid, cudaStream_t st);
+void real_sweep_launch_many(const RealProblem* d, int n, size_t smem, bool wide, int grid, int hasty, cudaStream_t st);
 
 // 2D grids of up to 64 x 64 points, one CTA a chain
 bool plane_sweep_supported(int Lx, int Ly);
@@ -101,9 +101,9 @@ void tile_string_launch(const RealProblem* d, int n, size_t smem, cudaStream_t s
 bool line_sweep_supported(int Lx);
 void line_sweep_launch(const RealProblem& p, cudaStream_t st);
 
-// polls before a barrier gives up, some ten seconds (PS_B200_BARRIER_POLLS=n: n, from
-// the sweep's construction on)
-constexpr int kBarrierPolls = 20000000;
+// polls before a barrier gives up, some ten seconds (PS_B200_BARRIER_GIVE_UP=1 at the
+// sweep's construction: at the first one in vain, for tests of what follows)
+constexpr long long kBarrierPolls = 20000000;
 
 // The work fields, operators and barrier words of one solve's sweep.
 class RealSweep {
@@ -128,7 +128,7 @@ public:
     // the chains'), throwing if so, and a new start after that
     bool failed() const;
     void check() const;
-    void reset(cudaStream_t st);
+    void reset();
 
 private:
     void init(const int n[3], const double k[3], double ds, int nl, bool os2);
@@ -139,7 +139,7 @@ private:
     double *work_ = nullptr, *frag_ = nullptr;
     unsigned* bar_ = nullptr;   // 32 words, then the error flag
     int* notice_ = nullptr;     // the error flag's copy in host memory (forms with barriers in memory)
-    int polls_ = kBarrierPolls;
+    int hasty_ = 0;
 };
 
 }  // namespace ps

@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(NT, PER_SM) tile_sweep_kernel(const __grid_con
             return true;
         }
         target += ncta;
-        return chain_barrier(p, bar, target);
+        return chain_barrier(bar, p.err, &p.notice, one.hasty, target);
     };
     for (int t = -1; t < p.Ns; t++) {
         if (t >= 0) {

@@ -1,5 +1,5 @@
 """A sweep that gives up at a grid barrier is reported by the calls that wait for its
-results, and by the next iteration, until fields are set again.  PS_B200_BARRIER_POLLS=0
+results, and by the next iteration, until fields are set again.  PS_B200_BARRIER_GIVE_UP=1
 lets a CTA give up as soon as it finds another one not yet there; every wait ends, and the
 context stays usable."""
 import numpy as np
@@ -32,7 +32,7 @@ def test_model_reports_it(ps, monkeypatch, dim, shape, cell):
     monkeypatch.setenv("PS_B200_AUTOTUNE", "0")
     c = ps.make_cell(dim, *cell)
     w = _fields(shape)
-    monkeypatch.setenv("PS_B200_BARRIER_POLLS", "0")
+    monkeypatch.setenv("PS_B200_BARRIER_GIVE_UP", "1")
     m = ps.ModelAB(dim, shape, c, (9, 13), 18.0, scft="Anderson", n_anderson=3)
     m.set_fields(w[0], w[1])
     m.update(2)
@@ -43,7 +43,7 @@ def test_model_reports_it(ps, monkeypatch, dim, shape, cell):
     for call in (lambda: m.grad_w(w[0], w[1]), m.stress):
         _given_up(ps, call)
         m.set_fields(w[0], w[1])
-    monkeypatch.delenv("PS_B200_BARRIER_POLLS")
+    monkeypatch.delenv("PS_B200_BARRIER_GIVE_UP")
     n = ps.ModelAB(dim, shape, c, (9, 13), 18.0, scft="Anderson", n_anderson=3)
     n.set_fields(w[0], w[1])
     n.update(2)
@@ -52,7 +52,7 @@ def test_model_reports_it(ps, monkeypatch, dim, shape, cell):
 
 def test_triblock_and_batch_report_it(ps, monkeypatch):
     monkeypatch.setenv("PS_B200_AUTOTUNE", "0")
-    monkeypatch.setenv("PS_B200_BARRIER_POLLS", "0")
+    monkeypatch.setenv("PS_B200_BARRIER_GIVE_UP", "1")
     dim, shape, cell = GRIDS[0]
     c = ps.make_cell(dim, *cell)
     w = _fields(shape, 3)
@@ -77,7 +77,7 @@ def test_triblock_and_batch_report_it(ps, monkeypatch):
 
 def test_updater_reports_it(ps, monkeypatch):
     import torch
-    monkeypatch.setenv("PS_B200_BARRIER_POLLS", "0")
+    monkeypatch.setenv("PS_B200_BARRIER_GIVE_UP", "1")
     dim, shape, cell = GRIDS[0]
     u = ps.RQM4(ps.make_cell(dim, *cell), *shape, 0.01)
     w = _fields(shape, 1)[0]
@@ -94,7 +94,7 @@ def test_updater_reports_it(ps, monkeypatch):
     torch.cuda.synchronize()
     _given_up(ps, lambda: u.solve(tq, tw))
     torch.cuda.synchronize()
-    monkeypatch.delenv("PS_B200_BARRIER_POLLS")
+    monkeypatch.delenv("PS_B200_BARRIER_GIVE_UP")
     v = ps.RQM4(ps.make_cell(dim, *cell), *shape, 0.01)
     out = v.solve(qs.copy(), w)
     v.check()
