@@ -332,10 +332,11 @@ void* ps_string_ab_stream(ps_string_ab* s);
  * (scft/polystring_AB_backThread.cc).  A batch holds n Model_AB solves,
  * each with its own parameters p[k] (RQM4; 2D or 3D grids with axis lengths
  * 16, 24, 32, 48, 64, 96 or 128; Ms, chiN, cell, EM or Anderson may all
- * differ).  Each line pass of contour step t is one launch over every solve
- * that has a step t; one batch iteration (= one Model_AB::update of every
- * solve) is one CUDA graph.  Results equal those of each solve run alone on
- * the per-pass path. */
+ * differ).  Solves on grids with a persistent sweep share sweep launches or
+ * have one each; on the others each line pass of contour step t is one launch
+ * over every solve that has a step t.  One batch iteration (= one
+ * Model_AB::update of every solve) is one CUDA graph.  Results equal those of
+ * each solve run alone. */
 typedef struct ps_batch_ab ps_batch_ab;
 int ps_batch_ab_create(const ps_model_ab_params* p, int n, ps_batch_ab** out);
 /* A batch of n Model_AB solves (members 0 .. n-1) and nq linear ABC

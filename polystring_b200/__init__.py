@@ -415,8 +415,9 @@ class BatchAB:
     ModelAB's constructor arguments (dim, shape, cell, Ms, chiN, lam, scft,
     n_anderson, compressible, contour; RQM4 only).  `triblocks` adds linear
     ABC solves (dicts of ModelABC's constructor arguments), numbered after
-    the AB solves.  update(n) runs n SCFT iterations of every solve; each line
-    pass of a contour step is one launch over all solves still running."""
+    the AB solves.  update(n) runs n SCFT iterations of every solve.  Solves on
+    grids with a persistent sweep share sweep launches or have one each; on the
+    others a line pass of a contour step is one launch over all still running."""
 
     def __init__(self, solves, triblocks=()):
         n, nq = len(solves), len(triblocks)

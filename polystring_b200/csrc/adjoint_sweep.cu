@@ -1,5 +1,5 @@
 // adjoint_sweep.cu -- the adjoint of the RQM4 chains on grids with a persistent
-// sweep (real_sweep.cu, plane_sweep.cu); adjoint.cu has the line-pass form.
+// sweep (real_sweep.cu, plane_sweep.cu, tile_sweep.cu); adjoint.cu has the line-pass form.
 //
 // Every split step S = e (.) D e (.) is symmetric, hence so is the RQM4 step
 // A = (4 S' S' - S) / 3, and lambda[t] = A lambda[t+1] + D[t] is the forward
@@ -27,7 +27,11 @@
 // no quotient by e', which is zero where w is large or infinite.)
 //
 // 48^3, Ns 128 (B200): the reverse sweeps took about 80 us a step and chain on
-// line passes (gradient 33.5 ms, stress 21.9 ms a call with the forward map).
+// line passes (gradient 33.5 ms, stress 21.9 ms a call with the forward map); the gradient
+// takes 4.5 ms now, of which the two sweeps 3.1 and the read-back of their kept fields 0.25
+// at 6.4 TB/s, and 32^3's stress (11.5 ms) 1.06, of which the sweep 0.73.  What bounds the
+// stress kernels is their registers, spilled from 24 points on at two CTAs an SM (56 bytes a
+// thread at 32 points, 756 at 64, 3100 at 128): 105 MB an axis at 2 TB/s.
 #include <algorithm>
 #include <cmath>
 #include <utility>
@@ -237,7 +241,7 @@ void stress_launch(const StressArgs& a, cudaStream_t st) {
 // for others and for the line passes' own.
 bool ModelAB::sweep_adjoint(bool grad) {
     if (!real_ || chain_->plan().naxes < 2) return false;
-    // the stress keeps an axis's operator in shared memory: 36 KB at 128 points, 250 KB at 352
+    // the stress keeps an axis's operator in shared memory: 32 KB at 128 points, 242 KB at 352
     if (!grad && (p_.Lx > 128 || p_.Ly > 128 || p_.Lz > 128)) return false;
     const size_t n = (size_t)Ns_ * M_;
     std::vector<std::pair<DevBuf*, size_t>> missing;

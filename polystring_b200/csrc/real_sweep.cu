@@ -30,7 +30,8 @@
 // plane, 40 % of the FP64 tensor peak while they run.  One CTA of 256 threads an SM:
 // with 255 registers each the next operands are prefetched; 512 threads spill, two
 // CTAs an SM gain nothing alone (19 to 20 us at 64^3), a barrier a field costs 10.2 us
-// at 32^3, two columns a lane 19.1 at 64^3.
+// at 32^3, two columns a lane 19.1 at 64^3.  The kernel spills 2.1 KB a thread, all of it
+// in the branches of 96 and 128 points; the one of shared launches, at 128 registers, 0.5 KB.
 //
 // Barriers (sweep_barrier.cuh) count arrivals per chain with a bounded spin; the launch
 // is cooperative, so all CTAs are resident.  On a timeout the CTA raises the error
@@ -661,6 +662,8 @@ void RealSweep::reset() {
     *((volatile int*)notice_) = 0;
 }
 
+// Single Model_AB solves are tuned.  Updaters, triblocks and batch members keep 8 columns,
+// the choice at most grids, rather than pay the timing at their construction.
 void RealSweep::tune(const RealProblem& p0, cudaStream_t st) {
     if (dim_ < 3) return;
     const char* force = getenv("PS_B200_SWEEP_VARIANT");

@@ -195,7 +195,8 @@ StringAB::StringAB(const ModelABParams& p, int m, int max_iter, int lo, int hi)
     chain_.reset(new PairChain(p.Lx, p.Ly, p.Lz, p.mde == 1 ? SCHEME_OS2 : SCHEME_RQM4, nloc_));
     // every image's chains in one launch of a persistent sweep per SCFT iteration
     // where the 2D grid has one (PS_B200_LINE_PASSES=1 keeps the batched line
-    // passes)
+    // passes): up to 64 x 64 a CTA a chain whatever the number of images, as batches
+    // past the clusters resident at once; clusters for fewer images are not measured
     const char* force = getenv("PS_B200_LINE_PASSES");
     const bool lines = force && force[0] == '1';
     if (!lines && p.Ly > 1 && p.Lz == 1 && (p.mde == 0 || cell_separable(p_.cell)) &&

@@ -1,6 +1,7 @@
-// tile_sweep.cu -- persistent RQM4 / OS2 sweep of 2D grids with an axis longer
-// than 64 points on real line operators (real_line.cuh): a CTA takes a tile of
-// eight lines, whose operators' products are dealt to its eight warps.
+// tile_sweep.cu -- persistent RQM4 / OS2 sweep of 2D grids on real line operators
+// (real_line.cuh): those with an axis longer than 64 points, and smaller ones where many
+// CTAs are faster than plane_sweep.cu's one a chain (RealSweep, BatchAB).  A CTA takes a
+// tile of eight lines, whose operators' products are dealt to its eight warps.
 //
 // Lx rows of Ly points, fields Z (half steps) and W (full step) of every chain
 // in global memory (L2).  A contour step is two phases with a barrier over the
