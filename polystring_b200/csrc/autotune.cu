@@ -80,7 +80,10 @@ void PairChain::autotune(cudaStream_t st) {
     const int nst = 2;
     const long M = M_;
     const long hstride = (long)(nst + 1) * M;
-    DevBuf hf((size_t)hstride * nbatch_), hc((size_t)hstride * nbatch_), ef((size_t)M * nbatch_);
+    DevBuf hf, hc, ef;   // the default tiles serve where the device has no room for them
+    if (!hf.try_alloc((size_t)hstride * nbatch_) || !hc.try_alloc((size_t)hstride * nbatch_) ||
+        !ef.try_alloc((size_t)M * nbatch_))
+        return;
     launch_fill(hf.p, hstride * nbatch_, 1.0, st);
     launch_fill(hc.p, hstride * nbatch_, 1.0, st);
     launch_fill(ef.p, M * nbatch_, 1.0, st);

@@ -649,7 +649,6 @@ double ModelAB::update_timed(int n, double* prop_ms) {
     PS_CUDA(cudaEventRecord(ev[2 * n + 1], st_));
     iter_ += n;
     PS_CUDA(cudaStreamSynchronize(st_));
-    check();
     double total = 0.0;
     for (int i = 0; i < n; i++) {
         float ms = 0.f;
@@ -659,6 +658,7 @@ double ModelAB::update_timed(int n, double* prop_ms) {
     float all = 0.f;
     PS_CUDA(cudaEventElapsedTime(&all, ev[2 * n], ev[2 * n + 1]));
     for (auto& e : ev) cudaEventDestroy(e);
+    check();
     *prop_ms = total;
     return all;
 }
