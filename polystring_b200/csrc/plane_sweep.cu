@@ -19,11 +19,12 @@
 // per line pass: 64^2 20).  So single solves leave it for the tiles of tile_sweep.cu
 // from 32 x 64 points on, while batches and strings, whose chains fill the SMs, stay.
 //
-// 1D: thread (chain, orbit) keeps the orbit's four points of q and the factors
+// 1D: thread (chain, orbit) keeps the orbit's four points of q and both factors
 // in registers; an operator's folded values go through shared memory, its
 // (block, output tile) products belong to one warp each, the two chains being
-// two of the eight lines of a product.  64 points 0.84 us a step (a launch a step: 10),
-// 128 1.6, 256 5.6; its chain of shared-memory trips bounds it.
+// two of the eight lines of a product.  64 points 0.82 us a step (a launch a step: 10),
+// 128 1.5, 256 5.6; its chain of shared-memory trips bounds it.  (e^{-w ds/2} as the square
+// of e^{-w ds/4}: 0.84, and three roundings for one.)
 #include <algorithm>
 
 #include "engine.h"
